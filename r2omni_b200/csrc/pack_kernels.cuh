@@ -276,55 +276,114 @@ __global__ void flush_ring_kernel(RingArgs r, int ring_tokens, int flush_tokens,
 }
 
 // ---------------------------------------------------------------------------
-// Normalised 128-point Walsh-Hadamard transform of 16-bit rows, fp32 butterflies in the reference's stage order
-// (stride 1, 2, ..., 64), result rounded to the element type.  One warp per row, four consecutive channels per
-// lane: two stages in registers, five through shuffles.  In place when out == in.
+// Row transforms: the normalised 128-point Walsh-Hadamard transform and the multimodal rotary embedding of 16-bit
+// rows of 128 channels.  fp32 arithmetic, butterflies in the reference's stage order (stride 1, 2, ..., 64), result
+// rounded to the element type.
+//
+// Eight lanes hold a row and a warp holds four: lane s of a row owns channels 8s..8s+7 and 64+8s..64+8s+7.  Loads and
+// stores are 16 bytes wide, the rotation's partner channel (d +- 64) and the butterflies of stride 1, 2, 4 and 64 are in
+// the lane's own registers, and only three stages go through shuffles (12 shuffle instructions a row; one row per
+// warp with four channels a lane took 24 and one table look-up per element).
 // ---------------------------------------------------------------------------
+struct Row16 { f32x2 x[8]; };   // channels (8s + e, 64 + 8s + e)
+
 template <bool BF16>
-__global__ void fwht128_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int64_t rows) {
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const uint2 raw = *reinterpret_cast<const uint2*>(in + row * 128 + 4 * lane);
-  float r[4];
-  if (BF16) {
-    r[0] = __uint_as_float(raw.x << 16); r[1] = __uint_as_float(raw.x & 0xffff0000u);
-    r[2] = __uint_as_float(raw.y << 16); r[3] = __uint_as_float(raw.y & 0xffff0000u);
-  } else {
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-    r[0] = a.x; r[1] = a.y; r[2] = b.x; r[3] = b.y;
+__device__ __forceinline__ void unpack8(const uint4& raw, float (&x)[8]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (BF16) {
+      x[2 * i] = __uint_as_float(w[i] << 16);
+      x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    } else {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+      x[2 * i] = f.x;
+      x[2 * i + 1] = f.y;
+    }
   }
-  const float a = __fadd_rn(r[0], r[1]), b = __fsub_rn(r[0], r[1]), c = __fadd_rn(r[2], r[3]), d = __fsub_rn(r[2], r[3]);
-  r[0] = __fadd_rn(a, c); r[1] = __fadd_rn(b, d); r[2] = __fsub_rn(a, c); r[3] = __fsub_rn(b, d);
+}
+template <bool BF16>
+__device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
+  uint4 v;
+  v.x = BF16 ? pack_bf16x2(x[0], x[1]) : pack_f16x2(x[0], x[1]);
+  v.y = BF16 ? pack_bf16x2(x[2], x[3]) : pack_f16x2(x[2], x[3]);
+  v.z = BF16 ? pack_bf16x2(x[4], x[5]) : pack_f16x2(x[4], x[5]);
+  v.w = BF16 ? pack_bf16x2(x[6], x[7]) : pack_f16x2(x[6], x[7]);
+  return v;
+}
+// 16 bytes at a pointer that is a multiple of 16 (wide) or of 8 bytes
+__device__ __forceinline__ uint4 load16(const uint16_t* p, bool wide) {
+  if (wide) return __ldcs(reinterpret_cast<const uint4*>(p));   // every row is touched once
+  const uint2 a = *reinterpret_cast<const uint2*>(p), b = *reinterpret_cast<const uint2*>(p + 4);
+  return make_uint4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void store16(uint16_t* p, const uint4& v, bool wide) {
+  if (wide) { __stcs(reinterpret_cast<uint4*>(p), v); return; }
+  *reinterpret_cast<uint2*>(p) = make_uint2(v.x, v.y);
+  *reinterpret_cast<uint2*>(p + 4) = make_uint2(v.z, v.w);
+}
+
+// The last stage (stride 64) is left to the caller's split_scaled: its operands are the two halves of a pair.
+__device__ __forceinline__ void hadamard_row(Row16& r, int s) {
+  const f32x2 minus = make_f32x2(-1.f, -1.f);
 #pragma unroll
-  for (int sft = 1; sft < 32; sft <<= 1) {
+  for (int span = 1; span < 8; span <<= 1) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float o = __shfl_xor_sync(0xffffffffu, r[e], sft);
-      r[e] = (lane & sft) ? __fsub_rn(o, r[e]) : __fadd_rn(r[e], o);
+    for (int e = 0; e < 8; ++e) {
+      if (e & span) continue;
+      const f32x2 a = r.x[e], b = r.x[e + span];
+      r.x[e] = add2(a, b);
+      r.x[e + span] = fma2(b, minus, a);   // a - b: the product is exact
     }
   }
 #pragma unroll
-  for (int e = 0; e < 4; ++e) r[e] = __fmul_rn(r[e], 0.08838834764831845f);
-  uint2 pk;
-  if (BF16) {
-    __nv_bfloat162 lo = __floats2bfloat162_rn(r[0], r[1]), hi = __floats2bfloat162_rn(r[2], r[3]);
-    pk.x = *reinterpret_cast<uint32_t*>(&lo); pk.y = *reinterpret_cast<uint32_t*>(&hi);
-  } else {
-    __half2 lo = __floats2half2_rn(r[0], r[1]), hi = __floats2half2_rn(r[2], r[3]);
-    pk.x = *reinterpret_cast<uint32_t*>(&lo); pk.y = *reinterpret_cast<uint32_t*>(&hi);
+  for (int sft = 1; sft < 8; sft <<= 1) {   // stride 8 * sft: own + other, or other - own
+    const float sign = (s & sft) ? -1.f : 1.f;
+    const f32x2 own = make_f32x2(sign, sign);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float lo, hi;
+      split_f32x2(r.x[e], lo, hi);
+      const f32x2 other = make_f32x2(__shfl_xor_sync(0xffffffffu, lo, sft), __shfl_xor_sync(0xffffffffu, hi, sft));
+      r.x[e] = fma2(r.x[e], own, other);
+    }
   }
-  *reinterpret_cast<uint2*>(out + row * 128 + 4 * lane) = pk;
+}
+__device__ __forceinline__ void split_row(const Row16& r, bool hadamard, float (&lo)[8], float (&hi)[8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    split_f32x2(r.x[e], lo[e], hi[e]);
+    if (hadamard) {
+      const f32x2 y = mul2(make_f32x2(__fadd_rn(lo[e], hi[e]), __fsub_rn(lo[e], hi[e])), make_f32x2(0.08838834764831845f, 0.08838834764831845f));
+      split_f32x2(y, lo[e], hi[e]);
+    }
+  }
 }
 
-// ---------------------------------------------------------------------------
-// Qwen multimodal rotary embedding of the query and key rows of a step, optionally followed by the 128-point
-// Hadamard transform, in one launch: row (request, head, token) of q or k, out[d] = x[d] * cos[axis(d)] +
-// rot(x)[d] * sin[axis(d)] with rot(x)[d] = -x[d + 64] (d < 64), x[d - 64] (d >= 64) and axis(d) chosen by the
-// section of d mod 64.  fp32 arithmetic, products and sum rounded separately (as the elementwise CPU form),
-// result rounded to the element type.  One warp per row, four consecutive channels per lane.
-// ---------------------------------------------------------------------------
+// In place when out == in.
+template <bool BF16>
+__global__ void __launch_bounds__(128) fwht128_kernel(const uint16_t* in, uint16_t* out, int64_t rows, bool wide) {
+  const int64_t row = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4 + ((threadIdx.x & 31) >> 3);
+  const int s = threadIdx.x & 7;
+  const bool valid = row < rows;   // every lane takes part in the shuffles
+  uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+  if (valid) { a = load16(in + row * 128 + 8 * s, wide); b = load16(in + row * 128 + 64 + 8 * s, wide); }
+  float lo[8], hi[8];
+  unpack8<BF16>(a, lo);
+  unpack8<BF16>(b, hi);
+  Row16 r;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) r.x[e] = make_f32x2(lo[e], hi[e]);
+  hadamard_row(r, s);
+  split_row(r, true, lo, hi);
+  if (!valid) return;
+  store16(out + row * 128 + 8 * s, pack8<BF16>(lo), wide);
+  store16(out + row * 128 + 64 + 8 * s, pack8<BF16>(hi), wide);
+}
+
+// Qwen multimodal rotary embedding of the query and key rows of a step, optionally followed by the Hadamard
+// transform, in one launch: row (request, head, token) of q or k, out[d] = x[d] * cos[axis(d)] + rot(x)[d] *
+// sin[axis(d)] with rot(x)[d] = -x[d + 64] (d < 64), x[d - 64] (d >= 64) and axis(d) chosen by the section of d mod 64.
 struct MropeArgs {
   const uint16_t* q; const uint16_t* k; uint16_t* q_out; uint16_t* k_out;
   const void* cos; const void* sin;
@@ -336,6 +395,9 @@ struct MropeArgs {
   const uint16_t* v; uint16_t* v_out;
   int64_t q_bstride, k_bstride, v_bstride;
   int v_hadamard;
+  int heads_per_warp;     // heads a warp walks with its tokens' table rows in registers
+  int wide;               // rows can be moved 16 bytes at a time
+  int table_vec;          // eight channels of a table row are one or two aligned 16-byte loads of one axis
 };
 
 __device__ __forceinline__ float load_rot(const void* base, int64_t index, int dtype) {
@@ -344,81 +406,102 @@ __device__ __forceinline__ float load_rot(const void* base, int64_t index, int d
   return dtype == R2K_DTYPE_BF16 ? __uint_as_float((uint32_t)raw << 16) : __half2float(__ushort_as_half(raw));
 }
 
+// Channels d0..d0+7 of one (request, token)'s table row; d0 is a multiple of 8.
+__device__ __forceinline__ void load_table8(const MropeArgs& a, const void* base, const int64_t (&stride)[4], int request,
+                                            int token, int d0, float (&x)[8]) {
+  const int64_t at = request * stride[1] + token * stride[2];
+  const int sd = d0 & 63;
+  if (a.table_vec) {
+    const int axis = sd < a.section0 ? 0 : (sd < a.section0 + a.section1 ? 1 : 2);
+    const int64_t i = at + axis * stride[0] + d0;
+    if (a.rot_dtype == 2) {
+      const float4 u = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i));
+      const float4 w = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i) + 1);
+      x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
+    } else {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + i));
+      if (a.rot_dtype == R2K_DTYPE_BF16) unpack8<true>(u, x); else unpack8<false>(u, x);
+    }
+    return;
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int axis = sd + e < a.section0 ? 0 : (sd + e < a.section0 + a.section1 ? 1 : 2);
+    x[e] = load_rot(base, at + axis * stride[0] + (d0 + e) * stride[3], a.rot_dtype);
+  }
+}
+
+// Bound by memory on a prefill: every row is read and written once, a (request, token)'s table rows are read once per
+// heads_per_warp rows.  A warp takes four consecutive (request, token)s and walks heads_per_warp heads with the next
+// head's rows in flight; blockIdx.y is the group of heads.  Twenty warps an SM at 94 registers: 16384 tokens of 16 + 2
+// heads with the Hadamard in 39 us (151 MB of rows, 3.9 TB/s; 36 us without it), from 139 us with a row per warp.
 template <bool BF16>
-__global__ void mrope_rows_kernel(MropeArgs a) {
+__global__ void __launch_bounds__(128, 5) mrope_rows_kernel(MropeArgs a) {
   // The decode launch that follows on the stream may start its CTAs and prefetch pool tiles right away (it is
   // launched with programmatic stream serialization); it reads the rows written here only after its own
   // dependency wait, i.e. after this grid has completed.
   launch_dependents();
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+  const int s = threadIdx.x & 7;
+  const int64_t n = (int64_t)a.batch * a.tokens;
+  const int64_t first = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4;
+  if (first >= n) return;
+  const int64_t i = first + ((threadIdx.x & 31) >> 3);
+  const bool valid = i < n;   // every lane takes part in the shuffles
+  const int request = (int)((valid ? i : first) / a.tokens), token = (int)((valid ? i : first) - (int64_t)request * a.tokens);
   const int heads = a.hq + a.hkv + (a.v != nullptr ? a.hkv : 0);
-  if (row >= (int64_t)a.batch * heads * a.tokens) return;
-  const int request = (int)(row / ((int64_t)heads * a.tokens));
-  const int local = (int)(row - (int64_t)request * heads * a.tokens);
-  const int head = local / a.tokens, token = local - head * a.tokens;
-  const int which = head < a.hq ? 0 : (head < a.hq + a.hkv ? 1 : 2);   // query, key or value row
-  const int h = which == 0 ? head : (which == 1 ? head - a.hq : head - a.hq - a.hkv);
-  const int nh = which == 0 ? a.hq : a.hkv;
-  const int64_t in_row = ((int64_t)h * a.tokens + token) * 128;
-  const int64_t off = (((int64_t)request * nh + h) * a.tokens + token) * 128;   // in the contiguous output
-  const uint16_t* src = which == 0 ? a.q + request * a.q_bstride : (which == 1 ? a.k + request * a.k_bstride : a.v + request * a.v_bstride);
-  uint16_t* dst = which == 0 ? a.q_out : (which == 1 ? a.k_out : a.v_out);
-  const uint2 raw = *reinterpret_cast<const uint2*>(src + in_row + 4 * lane);
-  if (which == 2 && !a.v_hadamard) {   // a value row that is only brought into place
-    *reinterpret_cast<uint2*>(dst + off + 4 * lane) = raw;
-    return;
-  }
-  float x[4];
-  if (BF16) {
-    x[0] = __uint_as_float(raw.x << 16); x[1] = __uint_as_float(raw.x & 0xffff0000u);
-    x[2] = __uint_as_float(raw.y << 16); x[3] = __uint_as_float(raw.y & 0xffff0000u);
-  } else {
-    const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-    const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-    x[0] = lo.x; x[1] = lo.y; x[2] = hi.x; x[3] = hi.y;
-  }
-  float r[4];
-  if (which == 2) {
+  const int h_begin = blockIdx.y * a.heads_per_warp, h_end = min(h_begin + a.heads_per_warp, heads);
+  // The next head's rows are in flight while one head's are worked on.
+  auto locate = [&](int head, const uint16_t*& src, uint16_t*& dst) {
+    const int which = head < a.hq ? 0 : (head < a.hq + a.hkv ? 1 : 2);   // query, key or value row
+    const int h = which == 0 ? head : (which == 1 ? head - a.hq : head - a.hq - a.hkv);
+    const int64_t in_row = ((int64_t)h * a.tokens + token) * 128 + 8 * s;
+    const int64_t out_row = (((int64_t)request * (which == 0 ? a.hq : a.hkv) + h) * a.tokens + token) * 128 + 8 * s;
+    src = (which == 0 ? a.q + request * a.q_bstride : which == 1 ? a.k + request * a.k_bstride : a.v + request * a.v_bstride) + in_row;
+    dst = (which == 0 ? a.q_out : which == 1 ? a.k_out : a.v_out) + out_row;
+  };
+  const uint16_t* src;
+  uint16_t* dst;
+  locate(h_begin, src, dst);
+  uint4 next_lo = load16(src, a.wide), next_hi = load16(src + 64, a.wide);
+  f32x2 cs[8];                   // cos of (d, d + 64)
+  float sin_lo[8], sin_hi[8];    // -sin of d (its partner enters negated), sin of d + 64
+  if (h_begin < a.hq + a.hkv) {
+    float lo[8], hi[8];
+    load_table8(a, a.cos, a.cos_stride, request, token, 8 * s, lo);
+    load_table8(a, a.cos, a.cos_stride, request, token, 64 + 8 * s, hi);
+    load_table8(a, a.sin, a.sin_stride, request, token, 8 * s, sin_lo);
+    load_table8(a, a.sin, a.sin_stride, request, token, 64 + 8 * s, sin_hi);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) r[e] = x[e];
-  } else {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int d = 4 * lane + e, sd = d & 63;
-      const float other = __shfl_xor_sync(0xffffffffu, x[e], 16);   // channel d +- 64 lives 16 lanes away
-      const float rotated = lane < 16 ? -other : other;
-      const int axis = sd < a.section0 ? 0 : (sd < a.section0 + a.section1 ? 1 : 2);
-      const float c = load_rot(a.cos, axis * a.cos_stride[0] + request * a.cos_stride[1] + token * a.cos_stride[2] + d * a.cos_stride[3],
-                               a.rot_dtype);
-      const float s = load_rot(a.sin, axis * a.sin_stride[0] + request * a.sin_stride[1] + token * a.sin_stride[2] + d * a.sin_stride[3],
-                               a.rot_dtype);
-      r[e] = __fmaf_rn(x[e], c, __fmul_rn(rotated, s));   // the reference's compiled form of x*cos + rot*sin: one product rounded, one fused
+    for (int e = 0; e < 8; ++e) { cs[e] = make_f32x2(lo[e], hi[e]); sin_lo[e] = -sin_lo[e]; }
+  }
+  for (int head = h_begin; head < h_end; ++head) {
+    const uint4 raw_lo = next_lo, raw_hi = next_hi;
+    uint16_t* const out = dst;
+    if (head + 1 < h_end) {
+      locate(head + 1, src, dst);
+      next_lo = load16(src, a.wide);
+      next_hi = load16(src + 64, a.wide);
     }
-  }
-  if (which == 2 || a.hadamard) {
-    const float p = __fadd_rn(r[0], r[1]), m = __fsub_rn(r[0], r[1]), c = __fadd_rn(r[2], r[3]), d = __fsub_rn(r[2], r[3]);
-    r[0] = __fadd_rn(p, c); r[1] = __fadd_rn(m, d); r[2] = __fsub_rn(p, c); r[3] = __fsub_rn(m, d);
-#pragma unroll
-    for (int sft = 1; sft < 32; sft <<= 1) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float o = __shfl_xor_sync(0xffffffffu, r[e], sft);
-        r[e] = (lane & sft) ? __fsub_rn(o, r[e]) : __fadd_rn(r[e], o);
-      }
+    const bool is_value = head >= a.hq + a.hkv;
+    if (is_value && !a.v_hadamard) {   // a value row that is only brought into place
+      if (valid) { store16(out, raw_lo, a.wide); store16(out + 64, raw_hi, a.wide); }
+      continue;
     }
+    float lo[8], hi[8];
+    unpack8<BF16>(raw_lo, lo);
+    unpack8<BF16>(raw_hi, hi);
+    Row16 x;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) r[e] = __fmul_rn(r[e], 0.08838834764831845f);
+    for (int e = 0; e < 8; ++e) {
+      x.x[e] = make_f32x2(lo[e], hi[e]);
+      // the reference's compiled form of x*cos + rot*sin: one product rounded, one fused
+      if (!is_value) x.x[e] = fma2(x.x[e], cs[e], make_f32x2(__fmul_rn(hi[e], sin_lo[e]), __fmul_rn(lo[e], sin_hi[e])));
+    }
+    const bool transform = is_value || a.hadamard;
+    if (transform) hadamard_row(x, s);
+    split_row(x, transform, lo, hi);
+    if (valid) { store16(out, pack8<BF16>(lo), a.wide); store16(out + 64, pack8<BF16>(hi), a.wide); }
   }
-  uint2 pk;
-  if (BF16) {
-    __nv_bfloat162 lo = __floats2bfloat162_rn(r[0], r[1]), hi = __floats2bfloat162_rn(r[2], r[3]);
-    pk.x = *reinterpret_cast<uint32_t*>(&lo); pk.y = *reinterpret_cast<uint32_t*>(&hi);
-  } else {
-    __half2 lo = __floats2half2_rn(r[0], r[1]), hi = __floats2half2_rn(r[2], r[3]);
-    pk.x = *reinterpret_cast<uint32_t*>(&lo); pk.y = *reinterpret_cast<uint32_t*>(&hi);
-  }
-  *reinterpret_cast<uint2*>(dst + off + 4 * lane) = pk;
 }
 
 }  // namespace r2k

@@ -264,6 +264,35 @@ int launch_pack_v2(const PackArgs& a, int batch, uint8_t* packed, void* scale, u
   return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
 }
 
+// Whether eight channels of a table row are whole aligned 16-byte words of one axis (see load_table8).
+bool table_vectorised(const void* base, const int64_t (&stride)[4], const MropeArgs& a) {
+  const int64_t unit = a.rot_dtype == 2 ? 4 : 8;   // elements of 16 bytes
+  return aligned16(base) && stride[3] == 1 && stride[0] % unit == 0 && stride[1] % unit == 0 && stride[2] % unit == 0 &&
+         a.section0 % 8 == 0 && a.section1 % 8 == 0;
+}
+
+int launch_mrope(MropeArgs& a, int32_t dtype, void* stream) {
+  DeviceInfo* dev;
+  const int rc = device_info(&dev);
+  if (rc) return rc;
+  a.wide = aligned16(a.q) && aligned16(a.k) && aligned16(a.q_out) && aligned16(a.k_out) && aligned16(a.v) && aligned16(a.v_out) &&
+           ((a.q_bstride | a.k_bstride | a.v_bstride) & 7) == 0;
+  a.table_vec = table_vectorised(a.cos, a.cos_stride, a) && table_vectorised(a.sin, a.sin_stride, a);
+  // Walking heads saves table reads, splitting them evens out the last wave: a warp takes the longest walk that still
+  // leaves two and a half waves of twenty warps for every SM (16384 tokens x 18 heads: 44.3 / 39.3 / 42.6 us with walks
+  // of 18 / 9 / 6 heads), and a decode step (a handful of tokens) one head per warp.
+  const int heads = a.hq + a.hkv + (a.v != nullptr ? a.hkv : 0);
+  const int64_t quads = ((int64_t)a.batch * a.tokens + 3) / 4;
+  const int64_t walks = quads * heads / ((int64_t)dev->sms * 50);
+  a.heads_per_warp = walks < 1 ? 1 : walks > heads ? heads : (int)walks;
+  const dim3 grid((unsigned)((quads + 3) / 4), (unsigned)((heads + a.heads_per_warp - 1) / a.heads_per_warp));
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (dtype == R2K_DTYPE_BF16) mrope_rows_kernel<true><<<grid, 128, 0, st>>>(a);
+  else mrope_rows_kernel<false><<<grid, 128, 0, st>>>(a);
+  ++g_launches;
+  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+}
+
 RingArgs ring_args(const R2KGeom* g, const R2KCacheView* v) {
   RingArgs r;
   r.recent_k = reinterpret_cast<uint8_t*>(v->recent_k);
@@ -701,12 +730,13 @@ int r2k_fwht128(const void* in, void* out, int32_t dtype, int64_t rows, void* st
   if (rows < 0 || (dtype != R2K_DTYPE_BF16 && dtype != R2K_DTYPE_FP16)) return R2K_ERR_GEOMETRY;
   if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 7u) return R2K_ERR_ALIGNMENT;
   if (rows == 0) return R2K_OK;
-  const unsigned grid = (unsigned)((rows + 3) / 4);
+  const unsigned grid = (unsigned)((rows + 15) / 16);
+  const bool wide = aligned16(in) && aligned16(out);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (dtype == R2K_DTYPE_BF16)
-    fwht128_kernel<true><<<grid, 128, 0, st>>>(reinterpret_cast<const uint16_t*>(in), reinterpret_cast<uint16_t*>(out), rows);
+    fwht128_kernel<true><<<grid, 128, 0, st>>>(reinterpret_cast<const uint16_t*>(in), reinterpret_cast<uint16_t*>(out), rows, wide);
   else
-    fwht128_kernel<false><<<grid, 128, 0, st>>>(reinterpret_cast<const uint16_t*>(in), reinterpret_cast<uint16_t*>(out), rows);
+    fwht128_kernel<false><<<grid, 128, 0, st>>>(reinterpret_cast<const uint16_t*>(in), reinterpret_cast<uint16_t*>(out), rows, wide);
   ++g_launches;
   return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
 }
@@ -732,13 +762,7 @@ int r2k_qk_mrope(const void* q, const void* k, void* q_out, void* k_out, int32_t
   a.section0 = section0; a.section1 = section1; a.rot_dtype = rot_dtype; a.hadamard = apply_hadamard ? 1 : 0;
   a.v = nullptr; a.v_out = nullptr; a.v_hadamard = 0; a.v_bstride = 0;
   a.q_bstride = (int64_t)num_q_heads * tokens * 128; a.k_bstride = (int64_t)num_kv_heads * tokens * 128;
-  const int64_t rows = (int64_t)batch * (num_q_heads + num_kv_heads) * tokens;
-  const unsigned grid = (unsigned)((rows + 3) / 4);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == R2K_DTYPE_BF16) mrope_rows_kernel<true><<<grid, 128, 0, st>>>(a);
-  else mrope_rows_kernel<false><<<grid, 128, 0, st>>>(a);
-  ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launch_mrope(a, dtype, stream);
 }
 
 int r2k_qkv_prologue(const void* q, int64_t q_bstride, const void* k, int64_t k_bstride, const void* v, int64_t v_bstride,
@@ -766,13 +790,7 @@ int r2k_qkv_prologue(const void* q, int64_t q_bstride, const void* k, int64_t k_
   a.batch = batch; a.hq = num_q_heads; a.hkv = num_kv_heads; a.tokens = 1;
   a.section0 = section0; a.section1 = section1; a.rot_dtype = rot_dtype;
   a.hadamard = key_hadamard ? 1 : 0; a.v_hadamard = value_hadamard ? 1 : 0;
-  const int64_t rows = (int64_t)batch * (num_q_heads + 2 * num_kv_heads);
-  const unsigned grid = (unsigned)((rows + 3) / 4);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == R2K_DTYPE_BF16) mrope_rows_kernel<true><<<grid, 128, 0, st>>>(a);
-  else mrope_rows_kernel<false><<<grid, 128, 0, st>>>(a);
-  ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launch_mrope(a, dtype, stream);
 }
 
 int r2k_append_recent(const R2KGeom* geom, const R2KCacheView* view, const R2KAppend* append, void* stream) {
