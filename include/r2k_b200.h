@@ -312,6 +312,37 @@ int r2k_pack_v_int2(const void* src, int32_t dtype, int32_t num_kv_heads, int64_
 int r2k_gather_rows(const void* src, int32_t num_kv_heads, int64_t src_rows, const int64_t* index,
                     int64_t count, void* dst, int64_t dst_rows, int64_t dst_start, void* stream);
 
+/*
+ * A whole cache from one layer's keys and values T [Hkv, rows, 128], in one launch: rows in pool order (bf16-value,
+ * INT4-value, INT2-value) packed as by the four calls above (same bits), token bookkeeping written, and everything
+ * behind the last used row of an arena set to its initial value.
+ * `pages`: the page table in pool order, evicted pages last, on the device: for page i the row of its first token in that
+ * order (`dst`) and in the source (`src`); n_pages + 1 entries, the last with dst = rows.  Every source row lies in exactly
+ * one page.  Token indices come either as one value per page (`global_base`, `logical_base`; a page's tokens are
+ * consecutive) or as one value per source row (`global_rows`, `logical_rows`).
+ * Replaces build_three_precision_cache's packing (r2omni/sspa/runtime/precision_pool.py:611-746, 787-984).
+ */
+typedef struct R2KPage { int32_t dst, src; } R2KPage;
+typedef struct R2KBuild {
+  const void* key; const void* value;
+  int64_t rows;
+  int32_t dtype, num_kv_heads, page_size, k_block, v2_group, n_pages;
+  int32_t n_fp, n_i4, n_i2, n_evicted;          /* tokens per pool; they add up to rows                     */
+  int32_t k_capacity, i2_capacity, recent_capacity, meta_capacity;   /* rows of the arenas; i64 entries of i2_global */
+  const R2KPage* pages;
+  const int64_t* global_base; const int64_t* logical_base;
+  const int64_t* global_rows; const int64_t* logical_rows;
+  uint8_t* k_packed; void* k_scale; uint8_t* k_zero;
+  void* fp_v;
+  uint8_t* i4_packed; float* i4_scale;
+  uint8_t* i2_packed; void* i2_scale; uint8_t* i2_zero;
+  void* recent_k; void* recent_v; int32_t* recent_len;
+  int64_t* recent_global; int64_t* recent_logical; int64_t* recent_page_lengths;
+  int64_t* fp_global; int64_t* fp_logical; int64_t* i4_global; int64_t* i4_logical;
+  int64_t* i2_global; int64_t* i2_logical; int64_t* evicted_global;
+} R2KBuild;
+int r2k_build_cache(const R2KBuild* build, void* stream);
+
 /* Normalised 128-point Walsh-Hadamard transform of `rows` 128-wide rows of the
  * given 16-bit type (fp32 butterflies, stages of stride 1..64, times 128^-1/2,
  * rounded to the element type); in place when out == in.  Replaces

@@ -1,0 +1,192 @@
+// Native host side of the operator API: what a Python caller pays for on every cache build.
+//
+// The work itself is behind the C ABI (r2k_b200.h); this module makes the tensors of a cache and fills the argument
+// block.  A cache build through Python and torch operators cost 1.3 ms of host time around 50 us of kernels, now 56 us in all.
+#include <ATen/EmptyTensor.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/extension.h>
+
+#include <cstring>
+#include <optional>
+#include <string>
+#include <vector>
+
+#include "r2k_b200.h"
+
+namespace {
+
+void check(int status, const char* what) {
+  if (status == R2K_OK) return;
+  const std::string message = std::string(what) + ": " + r2k_status_string(status);
+  if (status == R2K_ERR_GEOMETRY || status == R2K_ERR_ALIGNMENT || status == R2K_ERR_NULL || status == R2K_ERR_EMPTY)
+    throw py::value_error(message);
+  throw std::runtime_error(message);
+}
+
+int dtype_code(at::ScalarType t) {
+  if (t == at::kBFloat16) return R2K_DTYPE_BF16;
+  if (t == at::kHalf) return R2K_DTYPE_FP16;
+  throw py::value_error("the packed-KV path stores bfloat16 or float16 keys/values");
+}
+
+// ---------------------------------------------------------------------------
+// cache build
+// ---------------------------------------------------------------------------
+// The tensors of one cache share one allocation: offsets are handed out first, then the tensors are made over the storage.
+struct Slab {
+  struct Piece { at::ScalarType type; std::vector<int64_t> shape; int64_t offset; };
+  std::vector<Piece> pieces;
+  int64_t bytes = 0;
+  size_t add(at::ScalarType type, std::vector<int64_t> shape) {
+    int64_t n = (int64_t)c10::elementSize(type);
+    for (int64_t s : shape) n *= s;
+    pieces.push_back({type, std::move(shape), bytes});
+    bytes += (n + 255) / 256 * 256;
+    return pieces.size() - 1;
+  }
+  std::vector<at::Tensor> make(c10::Device device) {
+    at::Tensor base = at::empty({bytes > 0 ? bytes : 1}, at::TensorOptions().dtype(at::kByte).device(device));
+    std::vector<at::Tensor> out;
+    out.reserve(pieces.size());
+    for (const Piece& p : pieces) {
+      at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                                              c10::scalarTypeToTypeMeta(p.type));
+      t.unsafeGetTensorImpl()->set_storage_offset(p.offset / (int64_t)c10::elementSize(p.type));
+      t.unsafeGetTensorImpl()->set_sizes_contiguous(p.shape);
+      out.push_back(std::move(t));
+    }
+    return out;
+  }
+};
+
+at::Tensor host_i64(const at::Tensor& t) {
+  return t.device().is_cpu() && t.scalar_type() == at::kLong && t.is_contiguous() ? t : t.to(at::kCPU, at::kLong).contiguous();
+}
+
+inline int64_t ceil_to(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
+
+// Tier of a page class: 0 bf16, 1 INT4, 2 INT2 values, 3 evicted (precision_pool.py:611-669; classes of PageClass).
+inline int tier_of(int64_t cls) { return cls == 1 || cls == 3 || cls == 4 ? 0 : cls == 2 ? 1 : cls == 5 ? 2 : 3; }
+
+// build_three_precision_cache behind its argument checks.  Returns (tensors in the order of `names` on the Python side,
+// n_fp, n_i4, n_i2).
+py::tuple build_cache(const at::Tensor& key, const at::Tensor& value, const at::Tensor& page_classes, const at::Tensor& page_offsets,
+                      const at::Tensor& page_lengths, const at::Tensor& global_index, const at::Tensor& logical_position,
+                      int64_t page_size, int64_t k_block, int64_t v2_group, int64_t recent_capacity, int64_t append_capacity) {
+  const c10::cuda::CUDAGuard guard(key.device());
+  const int64_t h = key.size(0), rows = key.size(1), d = 128;
+  const int dtype = dtype_code(key.scalar_type());
+  const at::Tensor cls_t = host_i64(page_classes), off_t = host_i64(page_offsets), len_t = host_i64(page_lengths);
+  const int64_t n = cls_t.numel();
+  if (off_t.numel() != n || len_t.numel() != n) throw py::value_error("page table columns differ in length");
+  const int64_t *cls = cls_t.data_ptr<int64_t>(), *off = off_t.data_ptr<int64_t>(), *len = len_t.data_ptr<int64_t>();
+  int64_t tokens[4] = {0, 0, 0, 0}, total = 0;
+  for (int64_t i = 0; i < n; ++i) {
+    if (len[i] < 0 || off[i] < 0 || off[i] + len[i] > rows) throw py::value_error("page lies outside the keys and values");
+    tokens[tier_of(cls[i])] += len[i];
+    total += len[i];
+  }
+  if (total != rows) throw py::value_error("compact physical pools must cover every logical token");
+  if (rows > (int64_t)1 << 30) throw py::value_error("too many tokens for one cache");
+
+  // token bookkeeping: one value per page where a page's tokens are consecutive (the ordinary case), else whole arrays
+  at::Tensor global = global_index, logical = logical_position;
+  if (global.numel() < rows || logical.numel() < rows) throw py::value_error("token index arrays must cover every token");
+  bool by_page = global.device().is_cpu() && logical.device().is_cpu();
+  if (by_page) {
+    global = host_i64(global);
+    logical = host_i64(logical);
+    const int64_t *g = global.data_ptr<int64_t>(), *l = logical.data_ptr<int64_t>();
+    for (int64_t i = 0; i < n && by_page; ++i) {
+      const int64_t *gp = g + off[i], *lp = l + off[i];
+      int64_t odd = 0;
+      for (int64_t k = 1; k < len[i]; ++k) odd |= (gp[k] - gp[0] - k) | (lp[k] - lp[0] - k);
+      by_page = odd == 0;
+    }
+  }
+  // the page table in pool order: R2KPage x (n + 1), then the two bases
+  const int64_t words = (n + 1) + (by_page ? 2 * n : 0);
+  at::Tensor table_host = at::empty({words > 0 ? words : 1}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+  {
+    int64_t* w = table_host.data_ptr<int64_t>();
+    R2KPage* pages = reinterpret_cast<R2KPage*>(w);
+    static_assert(sizeof(R2KPage) == 8, "one table word");
+    int64_t *gb = w + n + 1, *lb = gb + n, at = 0, dst = 0;
+    const int64_t *g = by_page ? global.data_ptr<int64_t>() : nullptr, *l = by_page ? logical.data_ptr<int64_t>() : nullptr;
+    for (int tier = 0; tier < 4; ++tier)
+      for (int64_t i = 0; i < n; ++i) {
+        if (tier_of(cls[i]) != tier) continue;
+        pages[at] = R2KPage{(int32_t)dst, (int32_t)off[i]};
+        if (by_page) { gb[at] = len[i] > 0 ? g[off[i]] : 0; lb[at] = len[i] > 0 ? l[off[i]] : 0; }
+        dst += len[i];
+        ++at;
+      }
+    pages[n] = R2KPage{(int32_t)rows, 0};
+  }
+  const at::TensorOptions i64 = at::TensorOptions().dtype(at::kLong).device(key.device());
+  at::Tensor table = at::empty({table_host.numel()}, i64);
+  table.copy_(table_host, /*non_blocking=*/true);
+  if (!by_page) {
+    global = global.to(key.device(), at::kLong).contiguous();
+    logical = logical.to(key.device(), at::kLong).contiguous();
+  }
+
+  const int64_t n_fp = tokens[0], n_i4 = tokens[1], n_i2 = tokens[2], active = n_fp + n_i4 + n_i2;
+  const int64_t k_cap = std::max<int64_t>(128, ceil_to(active + append_capacity, 128)), i2_cap = std::max<int64_t>(128, ceil_to(n_i2 + append_capacity, 128));
+  const int64_t meta_cap = n_i2 + std::max<int64_t>(0, std::min(i2_cap - n_i2, k_cap - active)) / page_size * page_size;
+  const int64_t groups = d / v2_group;
+  const at::ScalarType T = key.scalar_type();
+  Slab slab;
+  slab.add(at::kByte, {1, h, k_cap, 64});
+  slab.add(at::kHalf, {1, h, k_cap / k_block, d});
+  slab.add(at::kByte, {1, h, k_cap / k_block, d});
+  slab.add(T, {1, h, n_fp, d});
+  slab.add(at::kByte, {1, h, n_i4, 64});
+  slab.add(at::kFloat, {1, h, n_i4, 1});
+  slab.add(at::kByte, {1, h, i2_cap, 32});
+  slab.add(at::kHalf, {1, h, i2_cap, groups, 1});
+  slab.add(at::kByte, {1, h, i2_cap, groups, 1});
+  slab.add(T, {1, h, recent_capacity, d});
+  slab.add(T, {1, h, recent_capacity, d});
+  slab.add(at::kInt, {1});
+  slab.add(at::kLong, {1, recent_capacity});
+  slab.add(at::kLong, {1, recent_capacity});
+  slab.add(at::kLong, {1, recent_capacity / page_size});
+  slab.add(at::kLong, {1, meta_cap});
+  slab.add(at::kLong, {1, meta_cap});
+  slab.add(at::kLong, {1, n_fp});
+  slab.add(at::kLong, {1, n_fp});
+  slab.add(at::kLong, {1, n_i4});
+  slab.add(at::kLong, {1, n_i4});
+  slab.add(at::kLong, {1, tokens[3]});
+  std::vector<at::Tensor> t = slab.make(key.device());
+  auto ptr = [&](size_t i) { return t[i].data_ptr(); };
+
+  R2KBuild b{};
+  b.key = key.data_ptr(); b.value = value.data_ptr();
+  b.rows = rows; b.dtype = dtype; b.num_kv_heads = (int32_t)h; b.page_size = (int32_t)page_size; b.k_block = (int32_t)k_block;
+  b.v2_group = (int32_t)v2_group; b.n_pages = (int32_t)n;
+  b.n_fp = (int32_t)n_fp; b.n_i4 = (int32_t)n_i4; b.n_i2 = (int32_t)n_i2; b.n_evicted = (int32_t)tokens[3];
+  b.k_capacity = (int32_t)k_cap; b.i2_capacity = (int32_t)i2_cap; b.recent_capacity = (int32_t)recent_capacity; b.meta_capacity = (int32_t)meta_cap;
+  int64_t* words_dev = table.data_ptr<int64_t>();
+  b.pages = reinterpret_cast<const R2KPage*>(words_dev);
+  if (by_page) { b.global_base = words_dev + n + 1; b.logical_base = words_dev + 2 * n + 1; }
+  else { b.global_rows = global.data_ptr<int64_t>(); b.logical_rows = logical.data_ptr<int64_t>(); }
+  b.k_packed = (uint8_t*)ptr(0); b.k_scale = ptr(1); b.k_zero = (uint8_t*)ptr(2);
+  b.fp_v = ptr(3); b.i4_packed = (uint8_t*)ptr(4); b.i4_scale = (float*)ptr(5);
+  b.i2_packed = (uint8_t*)ptr(6); b.i2_scale = ptr(7); b.i2_zero = (uint8_t*)ptr(8);
+  b.recent_k = ptr(9); b.recent_v = ptr(10); b.recent_len = (int32_t*)ptr(11);
+  b.recent_global = (int64_t*)ptr(12); b.recent_logical = (int64_t*)ptr(13); b.recent_page_lengths = (int64_t*)ptr(14);
+  b.i2_global = (int64_t*)ptr(15); b.i2_logical = (int64_t*)ptr(16);
+  b.fp_global = (int64_t*)ptr(17); b.fp_logical = (int64_t*)ptr(18); b.i4_global = (int64_t*)ptr(19); b.i4_logical = (int64_t*)ptr(20);
+  b.evicted_global = (int64_t*)ptr(21);
+  if (rows > 0) check(r2k_build_cache(&b, at::cuda::getCurrentCUDAStream().stream()), "r2k_build_cache");
+  return py::make_tuple(std::move(t), n_fp, n_i4, n_i2);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_r2k_host, m) {
+  m.def("build_cache", &build_cache);
+}

@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "device_utils.cuh"
+#include "r2k_b200.h"
 
 namespace r2k {
 
@@ -107,9 +108,56 @@ __global__ void __launch_bounds__(64) pack_k_int4_kernel(PackArgs a, uint8_t* pa
   zrow[2 * c + 1] = (uint8_t)zp1;
 }
 
-// ---- values: per-token symmetric INT4 -------------------------------------
-// One warp per (token, head, request); lane owns dims 4l..4l+3.
-// quantization.py:19-50, 77-102; fused_value_pack.py:25-70.
+// ---- values: one warp per (token, head, request), lane owns dims 4l..4l+3 ---
+template <bool BF16>
+__device__ __forceinline__ void unpack4(const uint2& w, float (&x)[4]) {
+  x[0] = raw_to_float<BF16>((uint16_t)(w.x & 0xffffu)); x[1] = raw_to_float<BF16>((uint16_t)(w.x >> 16));
+  x[2] = raw_to_float<BF16>((uint16_t)(w.y & 0xffffu)); x[3] = raw_to_float<BF16>((uint16_t)(w.y >> 16));
+}
+
+// Per-token symmetric INT4 (quantization.py:19-50, 77-102; fused_value_pack.py:25-70): returns the lane's two bytes.
+template <bool BF16>
+__device__ __forceinline__ uint16_t encode_v_int4(const uint2& w, float& sc) {
+  float x[4];
+  unpack4<BF16>(w, x);
+  float amax = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+  sc = fmaxf(__fdiv_rn(amax, 7.f), 1.0e-6f);
+  uint32_t out = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int q = (int)fminf(fmaxf(rintf(__fdiv_rn(x[e], sc)), -7.f), 7.f);
+    out |= (uint32_t)(q & 15) << (4 * e);
+  }
+  return (uint16_t)out;
+}
+
+// Per-token, per-group affine INT2 (int2_reference.py:96-151; fused_value_pack.py:72-149): returns the lane's byte;
+// `lanes` lanes (8, 16 or 32) share a group, its scale and its zero point.
+template <bool BF16>
+__device__ __forceinline__ uint8_t encode_v_int2(const uint2& w, int lanes, float& sc, float& zp) {
+  float x[4];
+  unpack4<BF16>(w, x);
+  float lo = fminf(fminf(x[0], x[1]), fminf(x[2], x[3]));
+  float hi = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+  for (int d = 1; d < lanes; d <<= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+  }
+  lo = fminf(lo, 0.f);
+  hi = fmaxf(hi, 0.f);
+  sc = fmaxf(__fdiv_rn(__fsub_rn(hi, lo), 3.f), 1.0e-6f);
+  zp = fminf(fmaxf(rintf(__fdiv_rn(-lo, sc)), 0.f), 3.f);
+  uint32_t out = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const uint32_t q = (uint32_t)fminf(fmaxf(rintf(__fadd_rn(__fdiv_rn(x[e], sc), zp)), 0.f), 3.f);
+    out |= q << (2 * e);
+  }
+  return (uint8_t)out;
+}
+
 template <bool BF16>
 __global__ void __launch_bounds__(128) pack_v_int4_kernel(PackArgs a, uint8_t* packed, float* scale, int64_t packed_bstride,
                                                           int64_t scale_bstride) {
@@ -119,27 +167,13 @@ __global__ void __launch_bounds__(128) pack_v_int4_kernel(PackArgs a, uint8_t* p
   const int64_t s = a.index ? a.index[i] : i;
   const uint16_t* src = reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(a.src) + req * a.src_bstride) +
                         ((int64_t)head * a.src_rows + s) * 128;
-  const uint2 w = *reinterpret_cast<const uint2*>(src + 4 * lane);
-  float x[4] = {raw_to_float<BF16>((uint16_t)(w.x & 0xffffu)), raw_to_float<BF16>((uint16_t)(w.x >> 16)),
-                raw_to_float<BF16>((uint16_t)(w.y & 0xffffu)), raw_to_float<BF16>((uint16_t)(w.y >> 16))};
-  float amax = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
-  const float sc = fmaxf(__fdiv_rn(amax, 7.f), 1.0e-6f);
-  uint32_t out = 0;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int q = (int)fminf(fmaxf(rintf(__fdiv_rn(x[e], sc)), -7.f), 7.f);
-    out |= (uint32_t)(q & 15) << (4 * e);
-  }
+  float sc;
+  const uint16_t out = encode_v_int4<BF16>(*reinterpret_cast<const uint2*>(src + 4 * lane), sc);
   const int64_t row = (int64_t)head * a.capacity + a.dst_start + i;
-  *reinterpret_cast<uint16_t*>(packed + req * packed_bstride + row * 64 + 2 * lane) = (uint16_t)out;
+  *reinterpret_cast<uint16_t*>(packed + req * packed_bstride + row * 64 + 2 * lane) = out;
   if (lane == 0) *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(scale) + req * scale_bstride + row * 4) = sc;
 }
 
-// ---- values: per-token, per-group affine INT2 ------------------------------
-// One warp per (token, head, request); lane owns dims 4l..4l+3 (one output byte).
-// int2_reference.py:96-151; fused_value_pack.py:72-149.
 template <bool BF16>
 __global__ void __launch_bounds__(128) pack_v_int2_kernel(PackArgs a, uint8_t* packed, __half* scale, uint8_t* zero,
                                                           int64_t packed_bstride, int64_t scale_bstride, int64_t zero_bstride,
@@ -151,31 +185,13 @@ __global__ void __launch_bounds__(128) pack_v_int2_kernel(PackArgs a, uint8_t* p
     const int64_t s = a.index ? a.index[i] : i;
     const uint16_t* src = reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(a.src) + req * a.src_bstride) +
                           ((int64_t)head * a.src_rows + s) * 128;
-    const uint2 w = *reinterpret_cast<const uint2*>(src + 4 * lane);
-    float x[4] = {raw_to_float<BF16>((uint16_t)(w.x & 0xffffu)), raw_to_float<BF16>((uint16_t)(w.x >> 16)),
-                  raw_to_float<BF16>((uint16_t)(w.y & 0xffffu)), raw_to_float<BF16>((uint16_t)(w.y >> 16))};
-    float lo = fminf(fminf(x[0], x[1]), fminf(x[2], x[3]));
-    float hi = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
     const int lanes = group / 4;  // lanes per group: 8, 16 or 32
-    for (int d = 1; d < lanes; d <<= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, d));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d));
-    }
-    lo = fminf(lo, 0.f);
-    hi = fmaxf(hi, 0.f);
-    const float sc = fmaxf(__fdiv_rn(__fsub_rn(hi, lo), 3.f), 1.0e-6f);
-    const float zp = fminf(fmaxf(rintf(__fdiv_rn(-lo, sc)), 0.f), 3.f);
-    uint32_t out = 0;
-  #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const uint32_t q = (uint32_t)fminf(fmaxf(rintf(__fadd_rn(__fdiv_rn(x[e], sc), zp)), 0.f), 3.f);
-      out |= q << (2 * e);
-    }
+    float sc, zp;
+    const uint8_t out = encode_v_int2<BF16>(*reinterpret_cast<const uint2*>(src + 4 * lane), lanes, sc, zp);
     const int64_t row = (int64_t)head * a.capacity + a.dst_start + i;
-    packed[req * packed_bstride + row * 32 + lane] = (uint8_t)out;
+    packed[req * packed_bstride + row * 32 + lane] = out;
     if ((lane & (lanes - 1)) == 0) {
-      const int groups = 128 / group;
-      const int64_t m = row * groups + lane / lanes;
+      const int64_t m = row * (128 / group) + lane / lanes;
       reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(scale) + req * scale_bstride)[m] = __float2half_rn(sc);
       zero[req * zero_bstride + m] = (uint8_t)zp;
     }

@@ -6,6 +6,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "build_kernel.cuh"
 #include "decode_kernel.cuh"
 #include "pack_kernels.cuh"
 #include "r2k_b200.h"
@@ -721,6 +722,63 @@ int r2k_gather_rows(const void* src, int32_t num_kv_heads, int64_t src_rows, con
   dim3 grid((unsigned)((count + 3) / 4), (unsigned)num_kv_heads, 1);
   gather_rows_kernel<<<grid, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const uint16_t*>(src), src_rows, index, count, reinterpret_cast<uint16_t*>(dst), dst_rows, dst_start);
+  ++g_launches;
+  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+}
+
+int r2k_build_cache(const R2KBuild* build, void* stream) {
+  if (build == nullptr) return R2K_ERR_NULL;
+  const R2KBuild& b = *build;
+  if ((b.rows > 0 && (!b.key || !b.value)) || !b.pages || !b.k_packed || !b.k_scale || !b.k_zero || !b.i2_packed || !b.i2_scale || !b.i2_zero ||
+      !b.recent_k || !b.recent_v || !b.recent_len || !b.recent_global || !b.recent_logical || !b.recent_page_lengths)
+    return R2K_ERR_NULL;
+  if ((b.n_fp && (!b.fp_v || !b.fp_global || !b.fp_logical)) || (b.n_i4 && (!b.i4_packed || !b.i4_scale || !b.i4_global || !b.i4_logical)) ||
+      (b.meta_capacity && (!b.i2_global || !b.i2_logical)) || (b.n_evicted && !b.evicted_global))
+    return R2K_ERR_NULL;
+  if (!b.global_rows != !b.logical_rows || (!b.global_rows && (!b.global_base || !b.logical_base))) return R2K_ERR_NULL;
+  if (b.dtype != R2K_DTYPE_BF16 && b.dtype != R2K_DTYPE_FP16) return R2K_ERR_GEOMETRY;
+  if (b.num_kv_heads < 1 || b.n_pages < 0 || (b.n_pages == 0 && b.rows != 0) || b.rows < 0 || b.rows > (int64_t)1 << 30) return R2K_ERR_GEOMETRY;
+  if (!pow2_in(b.k_block, 32, 64, 128) || !pow2_in(b.v2_group, 32, 64, 128) || !pow2_in(b.page_size, 16, 32, 64)) return R2K_ERR_GEOMETRY;
+  if (b.n_fp < 0 || b.n_i4 < 0 || b.n_i2 < 0 || b.n_evicted < 0 || (int64_t)b.n_fp + b.n_i4 + b.n_i2 + b.n_evicted != b.rows)
+    return R2K_ERR_GEOMETRY;
+  if (b.k_capacity % 128 || b.recent_capacity % b.page_size || b.recent_capacity < 1) return R2K_ERR_GEOMETRY;
+  if (b.k_capacity < b.n_fp + b.n_i4 + b.n_i2 || b.i2_capacity < b.n_i2 || b.meta_capacity < b.n_i2) return R2K_ERR_CAPACITY;
+  if (!aligned16(b.k_packed) || !aligned16(b.k_scale) || !aligned16(b.k_zero) || !aligned16(b.fp_v) || !aligned16(b.i4_packed) ||
+      ((reinterpret_cast<uintptr_t>(b.key) | reinterpret_cast<uintptr_t>(b.value)) & 7u))
+    return R2K_ERR_ALIGNMENT;
+  BuildArgs a;
+  a.b = b;
+  a.active = b.n_fp + b.n_i4 + b.n_i2;
+  a.chunks = (a.active + kBuildRows - 1) / kBuildRows;
+  a.chunk_ctas = a.chunks * b.num_kv_heads;
+  a.meta_ctas = (int)((b.rows + kBuildThreads - 1) / kBuildThreads);
+  a.n_fills = 0;
+  int64_t ctas = (int64_t)a.chunk_ctas + a.meta_ctas;
+  auto fill = [&](void* base, int64_t from, int64_t to, int64_t unit, int heads, int value) {   // units [from, to) of every head's `to`
+    if (from >= to) return;
+    a.fill[a.n_fills++] = BuildFill{static_cast<uint8_t*>(base) + from * unit, to * unit, (to - from) * unit, heads, value};
+    ctas += ((to - from) * unit + kFillBytes - 1) / kFillBytes * heads;
+  };
+  const int h = b.num_kv_heads, g2 = 128 / b.v2_group;
+  const int64_t blocks = (a.active + b.k_block - 1) / b.k_block, block_cap = b.k_capacity / b.k_block;
+  fill(b.k_packed, a.active, b.k_capacity, 64, h, 0);
+  fill(b.k_scale, blocks, block_cap, 256, h, 0);
+  fill(b.k_zero, blocks, block_cap, 128, h, 0);
+  fill(b.i2_packed, b.n_i2, b.i2_capacity, 32, h, 0);
+  fill(b.i2_scale, b.n_i2, b.i2_capacity, 2 * g2, h, 0);
+  fill(b.i2_zero, b.n_i2, b.i2_capacity, g2, h, 0);
+  fill(b.recent_k, 0, b.recent_capacity, 256, h, 0);
+  fill(b.recent_v, 0, b.recent_capacity, 256, h, 0);
+  fill(b.recent_global, 0, b.recent_capacity, 8, 1, 0xFF);
+  fill(b.recent_logical, 0, b.recent_capacity, 8, 1, 0xFF);
+  fill(b.i2_global, b.n_i2, b.meta_capacity, 8, 1, 0xFF);
+  fill(b.i2_logical, b.n_i2, b.meta_capacity, 8, 1, 0xFF);
+  fill(b.recent_page_lengths, 0, b.recent_capacity / b.page_size, 8, 1, 0);
+  static_assert(kMaxFills == 13, "one per call above");
+  if (ctas > 0x7fffffff) return R2K_ERR_GEOMETRY;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (b.dtype == R2K_DTYPE_BF16) build_cache_kernel<true><<<(unsigned)ctas, kBuildThreads, 0, st>>>(a);
+  else build_cache_kernel<false><<<(unsigned)ctas, kBuildThreads, 0, st>>>(a);
   ++g_launches;
   return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
 }

@@ -18,6 +18,7 @@ from typing import Literal
 import torch
 
 from .. import _lib as L
+from .._host import host
 
 
 class PageClass(IntEnum):
@@ -73,48 +74,6 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 def _ptr(t: torch.Tensor | None):
     return None if t is None or t.numel() == 0 else C.c_void_p(t.data_ptr())
-
-
-# --------------------------------------------------------------------------- #
-# pack routines (C ABI)
-# --------------------------------------------------------------------------- #
-def pack_k_int4_into(src, index, packed, scale, zero, *, k_block: int, dst_start: int) -> None:
-    """Quantise ``src[:, index]`` ([H,S,128]) into key-arena rows starting at
-    ``dst_start`` (compact_int4_key.py:83-110, 200-220)."""
-    h, rows, _ = src.shape
-    count = int(rows if index is None else index.numel())
-    L.check(L.lib().r2k_pack_k_int4(
-        _ptr(src), dtype_code(src.dtype), h, C.c_int64(rows), _ptr(index), C.c_int64(count),
-        _ptr(packed), _ptr(scale), _ptr(zero), C.c_int64(packed.shape[-2]), k_block, C.c_int64(dst_start),
-        C.c_void_p(_stream_ptr(src.device))), "r2k_pack_k_int4")
-
-
-def pack_v_int4_into(src, index, packed, scale, *, dst_start: int) -> None:
-    """fused_value_pack.py:25-70 / quantization.py:19-50."""
-    h, rows, _ = src.shape
-    count = int(rows if index is None else index.numel())
-    L.check(L.lib().r2k_pack_v_int4(
-        _ptr(src), dtype_code(src.dtype), h, C.c_int64(rows), _ptr(index), C.c_int64(count),
-        _ptr(packed), _ptr(scale), C.c_int64(packed.shape[-2]), C.c_int64(dst_start),
-        C.c_void_p(_stream_ptr(src.device))), "r2k_pack_v_int4")
-
-
-def pack_v_int2_into(src, index, packed, scale, zero, *, group: int, dst_start: int) -> None:
-    """fused_value_pack.py:72-149 / int2_reference.py:96-151."""
-    h, rows, _ = src.shape
-    count = int(rows if index is None else index.numel())
-    L.check(L.lib().r2k_pack_v_int2(
-        _ptr(src), dtype_code(src.dtype), h, C.c_int64(rows), _ptr(index), C.c_int64(count),
-        _ptr(packed), _ptr(scale), _ptr(zero), C.c_int64(packed.shape[-2]), group, C.c_int64(dst_start),
-        C.c_void_p(_stream_ptr(src.device))), "r2k_pack_v_int2")
-
-
-def gather_rows_into(src, index, dst, *, dst_start: int = 0) -> None:
-    h, rows, _ = src.shape
-    count = int(index.numel())
-    L.check(L.lib().r2k_gather_rows(
-        _ptr(src), h, C.c_int64(rows), _ptr(index), C.c_int64(count), _ptr(dst), C.c_int64(dst.shape[-2]),
-        C.c_int64(dst_start), C.c_void_p(_stream_ptr(src.device))), "r2k_gather_rows")
 
 
 # --------------------------------------------------------------------------- #
@@ -616,6 +575,12 @@ def tier_sorted_tokens(plan: LayerCompressionPlan):
     return tuple(tokens[token_tier == t] for t in range(4))
 
 
+# the tensors host().build_cache returns, in order
+_BUILT = ("k_packed", "k_scale", "k_zero", "fp_v", "i4_packed", "i4_scale", "i2_packed", "i2_scale", "i2_zero", "recent_k", "recent_v",
+          "recent_len_device", "recent_global", "recent_logical", "recent_page_lengths", "i2_global", "i2_logical", "fp_global",
+          "fp_logical", "i4_global", "i4_logical", "evicted_global")
+
+
 def build_three_precision_cache(
     key: torch.Tensor,
     value: torch.Tensor,
@@ -665,67 +630,17 @@ def build_three_precision_cache(
     if not key.is_cuda:
         raise RuntimeError("build_three_precision_cache packs on a CUDA device; there is no CPU path")
     dtype_code(key.dtype)
-    dev = key.device
-    key, value = key.contiguous(), value.contiguous()
-    h, s, d = key.shape
-
-    fp_t, i4_t, i2_t, ev_t = tier_sorted_tokens(plan)
-    if fp_t.numel() + i4_t.numel() + i2_t.numel() + ev_t.numel() != s:
-        raise ValueError("compact physical pools must cover every logical token")
     append_capacity = plan.recent_fp_capacity if compact_key_append_capacity is None else int(compact_key_append_capacity)
-    n_fp, n_i4, n_i2 = int(fp_t.numel()), int(i4_t.numel()), int(i2_t.numel())
+    # page table, allocation, packing and token bookkeeping: native, one launch (csrc/host_ext.cpp, csrc/build_kernel.cuh)
+    tensors, n_fp, n_i4, n_i2 = host().build_cache(
+        key.contiguous(), value.contiguous(), plan.page_classes, plan.page_offsets, plan.page_lengths, plan.global_token_indices,
+        plan.logical_positions, int(page_size), int(key_quantization_superblock), int(int2_group_size),
+        int(plan.recent_fp_capacity), append_capacity)
     active = n_fp + n_i4 + n_i2
-    k_cap = max(128, _ceil_to(active + append_capacity, 128))
-    i2_cap = max(128, _ceil_to(n_i2 + append_capacity, 128))
-    groups = d // int2_group_size
-    cap = int(plan.recent_fp_capacity)
-    glob = plan.global_token_indices.detach().cpu().long()
-    logi = plan.logical_positions.detach().cpu().long()
-    meta_cap = n_i2 + max(0, min(i2_cap - n_i2, k_cap - active)) // page_size * page_size
-
-    def z(*shape, dtype):
-        return torch.zeros((1, *shape), device=dev, dtype=dtype)
-
-    def meta(src, extra=0):
-        out = torch.full((1, src.numel() + extra), -1, device=dev, dtype=torch.long)
-        out[0, : src.numel()] = src.to(dev)
-        return out
-
-    arenas = PackedArenas(
+    return ThreePrecisionCache(PackedArenas(
         dtype=key.dtype, page_size=int(page_size), k_block=int(key_quantization_superblock), v2_group=int(int2_group_size),
-        flush=int(recent_flush_size),
-        k_packed=z(h, k_cap, 64, dtype=torch.uint8),
-        k_scale=z(h, k_cap // key_quantization_superblock, d, dtype=torch.float16),
-        k_zero=z(h, k_cap // key_quantization_superblock, d, dtype=torch.uint8),
-        k_active=active, k_offsets=(0, n_fp, n_fp + n_i4),
-        fp_v=z(h, n_fp, d, dtype=key.dtype),
-        i4_packed=z(h, n_i4, 64, dtype=torch.uint8), i4_scale=z(h, n_i4, 1, dtype=torch.float32),
-        i2_packed=z(h, i2_cap, 32, dtype=torch.uint8), i2_scale=z(h, i2_cap, groups, 1, dtype=torch.float16),
-        i2_zero=z(h, i2_cap, groups, 1, dtype=torch.uint8), i2_active=n_i2,
-        recent_k=z(h, cap, d, dtype=key.dtype), recent_v=z(h, cap, d, dtype=key.dtype),
-        recent_len_device=torch.zeros(1, device=dev, dtype=torch.int32),
-        recent_global=torch.full((1, cap), -1, device=dev, dtype=torch.long),
-        recent_logical=torch.full((1, cap), -1, device=dev, dtype=torch.long),
-        recent_page_lengths=torch.zeros((1, cap // page_size), device=dev, dtype=torch.long),
-        recent_len=0,
-        i2_global=meta(glob[i2_t], meta_cap - n_i2), i2_logical=meta(logi[i2_t], meta_cap - n_i2),
-        fp_global=meta(glob[fp_t]), fp_logical=meta(logi[fp_t]),
-        i4_global=meta(glob[i4_t]), i4_logical=meta(logi[i4_t]),
-        evicted_global=meta(glob[ev_t]),
-        generated_k_offset=active, static_i2_tokens=n_i2,
-    )
-    if active:
-        order = torch.cat((fp_t, i4_t, i2_t)).to(dev)
-        pack_k_int4_into(key, order, arenas.k_packed[0], arenas.k_scale[0], arenas.k_zero[0],
-                         k_block=arenas.k_block, dst_start=0)
-    if n_fp:
-        gather_rows_into(value, fp_t.to(dev), arenas.fp_v[0])
-    if n_i4:
-        pack_v_int4_into(value, i4_t.to(dev), arenas.i4_packed[0], arenas.i4_scale[0], dst_start=0)
-    if n_i2:
-        pack_v_int2_into(value, i2_t.to(dev), arenas.i2_packed[0], arenas.i2_scale[0], arenas.i2_zero[0],
-                         group=arenas.v2_group, dst_start=0)
-    return ThreePrecisionCache(arenas)
+        flush=int(recent_flush_size), k_active=active, k_offsets=(0, n_fp, n_fp + n_i4), i2_active=n_i2, recent_len=0,
+        generated_k_offset=active, static_i2_tokens=n_i2, **dict(zip(_BUILT, tensors))))
 
 
 def adopt_reference_cache(cache) -> ThreePrecisionCache:
