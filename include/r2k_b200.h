@@ -41,6 +41,7 @@ enum {
   R2K_FLAG_OUTPUT_HADAMARD = 1, /* round to the element type, then 128-point orthonormal WHT
                                    (r2omni/sspa/kernels/triton_fourq_splitk.py:999-1005)   */
   R2K_FLAG_OUT_F32 = 2,         /* `out` is float32 [B,Hq,128] instead of the element type  */
+  R2K_FLAG_OUT_BF16 = 8,        /* `out` is bf16 [B,Hq,128] whatever the element type        */
   R2K_FLAG_OUT_STATE = 4        /* `out` is float32 [B,Hq,130]: (max, sum-exp, un-normalised
                                    weighted V[128]) in natural-log units, for cross-shard merge */
 };

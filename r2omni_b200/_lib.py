@@ -8,7 +8,7 @@ from .build import LIB
 
 OK, ERR_NULL, ERR_GEOMETRY, ERR_ALIGNMENT, ERR_CAPACITY, ERR_WORKSPACE, ERR_CUDA, ERR_DEVICE_TIMEOUT, ERR_EMPTY = range(9)
 DTYPE_BF16, DTYPE_FP16 = 0, 1
-FLAG_OUTPUT_HADAMARD, FLAG_OUT_F32, FLAG_OUT_STATE = 1, 2, 4
+FLAG_OUTPUT_HADAMARD, FLAG_OUT_F32, FLAG_OUT_STATE, FLAG_OUT_BF16 = 1, 2, 4, 8
 
 EXPORTS = (
     "r2k_status_string", "r2k_launch_count", "r2k_decode_workspace_bytes", "r2k_decode_workspace_init", "r2k_decode",

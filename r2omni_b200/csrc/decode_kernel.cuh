@@ -323,7 +323,7 @@ __device__ __forceinline__ void write_output(const DecodeParams& p, size_t orow,
     *reinterpret_cast<float4*>(o + 4) = make_float4(r[4], r[5], r[6], r[7]);
   } else {
     uint4 pk;
-    if (BF16) { pk.x = pack_bf16x2(r[0], r[1]); pk.y = pack_bf16x2(r[2], r[3]); pk.z = pack_bf16x2(r[4], r[5]); pk.w = pack_bf16x2(r[6], r[7]); }
+    if (BF16 || (p.flags & R2K_FLAG_OUT_BF16)) { pk.x = pack_bf16x2(r[0], r[1]); pk.y = pack_bf16x2(r[2], r[3]); pk.z = pack_bf16x2(r[4], r[5]); pk.w = pack_bf16x2(r[6], r[7]); }
     else { pk.x = pack_f16x2(r[0], r[1]); pk.y = pack_f16x2(r[2], r[3]); pk.z = pack_f16x2(r[4], r[5]); pk.w = pack_f16x2(r[6], r[7]); }
     *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + orow * kD + 8 * sub) = pk;
   }
@@ -877,7 +877,7 @@ __global__ void merge_states_kernel(const float* __restrict__ states, int num_st
     *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + (int64_t)row * kD + 4 * lane) = make_float4(r[0], r[1], r[2], r[3]);
   } else {
     uint2 pk;
-    if (bf16) { pk.x = pack_bf16x2(r[0], r[1]); pk.y = pack_bf16x2(r[2], r[3]); }
+    if (bf16 || (flags & R2K_FLAG_OUT_BF16)) { pk.x = pack_bf16x2(r[0], r[1]); pk.y = pack_bf16x2(r[2], r[3]); }
     else { pk.x = pack_f16x2(r[0], r[1]); pk.y = pack_f16x2(r[2], r[3]); }
     *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(out) + (int64_t)row * kD + 4 * lane) = pk;
   }

@@ -1,7 +1,8 @@
-// Native host side of the operator API: what a Python caller pays for on every cache build.
+// Native host side of the operator API: what a Python caller pays for on every decode step and on every cache build.
 //
-// The work itself is behind the C ABI (r2k_b200.h); this module makes the tensors of a cache and fills the argument
-// block.  A cache build through Python and torch operators cost 1.3 ms of host time around 50 us of kernels, now 56 us in all.
+// The work itself is behind the C ABI (r2k_b200.h); this module checks torch tensors, makes the tensors of a cache and
+// fills the argument blocks.  A decode step through Python and ctypes cost 5.4 us of host time (7.0 with an append) around a
+// launch that takes 2.2, a cache build 1.3 ms around 50 us of kernels.
 #include <ATen/EmptyTensor.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -29,6 +30,57 @@ int dtype_code(at::ScalarType t) {
   if (t == at::kHalf) return R2K_DTYPE_FP16;
   throw py::value_error("the packed-KV path stores bfloat16 or float16 keys/values");
 }
+
+// ---------------------------------------------------------------------------
+// decode step
+// ---------------------------------------------------------------------------
+// Everything about an executor's launch that does not change from step to step.  The geometry and view structs are the ones
+// the Python side holds (and keeps alive); the output tensor is the workspace's.
+struct Step {
+  R2KGeom* geom;
+  const R2KCacheView* view;
+  void* workspace;
+  size_t workspace_bytes;
+  at::Tensor output;
+  at::ScalarType dtype;
+  c10::Device device;
+  uint32_t flags;
+  int64_t batch, heads, kv_numel;
+
+  Step(uintptr_t geom_, uintptr_t view_, const at::Tensor& buffer, const at::Tensor& output_, const at::Tensor& like, uint32_t flags_)
+      : geom(reinterpret_cast<R2KGeom*>(geom_)), view(reinterpret_cast<const R2KCacheView*>(view_)), workspace(buffer.data_ptr()),
+        workspace_bytes((size_t)buffer.numel()), output(output_), dtype(like.scalar_type()), device(like.device()), flags(flags_),
+        batch(geom->batch), heads(geom->num_q_heads), kv_numel((int64_t)geom->batch * geom->num_kv_heads * 128) {}
+
+  // ap filled from (k, v); the indices are the caller's business
+  void rows(R2KAppend& ap, const at::Tensor& k, const at::Tensor& v) const {
+    if (k.numel() != kv_numel || v.numel() != kv_numel || k.device() != device || v.device() != device || !k.is_contiguous() ||
+        !v.is_contiguous() || k.scalar_type() != dtype || v.scalar_type() != dtype)
+      throw py::value_error("append K/V must be contiguous [B,Hkv,1,D] or [B,Hkv,D]");
+    ap.k = k.data_ptr();
+    ap.v = v.data_ptr();
+  }
+
+  void launch(const at::Tensor& query, const R2KAppend* ap, int32_t n_i2) {
+    const bool four = query.dim() == 4 && query.size(2) == 1;   // [B,Hq,1,128]
+    if (!((query.dim() == 3 && query.size(2) == 128) || (four && query.size(3) == 128)) || query.size(0) != batch ||
+        query.size(1) != heads || query.device() != device || query.scalar_type() != dtype || !query.is_contiguous())
+      throw py::value_error("query does not match prepared split-K executor");
+    geom->n_i2 = n_i2;   // the only extent that moves during generation (flushes)
+    const int status = r2k_decode(geom, view, query.data_ptr(), ap, workspace, workspace_bytes, output.data_ptr(), flags,
+                                  at::cuda::getCurrentCUDAStream(device.index()).stream());
+    if (status != R2K_OK) check(status, "r2k_decode");
+  }
+  void plain(const at::Tensor& query, int32_t n_i2) { launch(query, nullptr, n_i2); }
+  void append(const at::Tensor& query, const at::Tensor& k, const at::Tensor& v, int64_t global_index, int64_t logical_position,
+                    int32_t n_i2) {
+    R2KAppend ap{};
+    rows(ap, k, v);
+    ap.global_index = global_index;
+    ap.logical_position = logical_position;
+    launch(query, &ap, n_i2);
+  }
+};
 
 // ---------------------------------------------------------------------------
 // cache build
@@ -188,5 +240,9 @@ py::tuple build_cache(const at::Tensor& key, const at::Tensor& value, const at::
 }  // namespace
 
 PYBIND11_MODULE(_r2k_host, m) {
+  py::class_<Step>(m, "Step")
+      .def(py::init<uintptr_t, uintptr_t, const at::Tensor&, const at::Tensor&, const at::Tensor&, uint32_t>())
+      .def("plain", &Step::plain)
+      .def("append", &Step::append);
   m.def("build_cache", &build_cache);
 }

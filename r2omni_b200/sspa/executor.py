@@ -16,6 +16,7 @@ from typing import Sequence
 import torch
 
 from .. import _lib as L
+from .._host import host
 from .cache import PackedArenas, ThreePrecisionCache, _stream_ptr, dtype_code, stack_arenas
 
 
@@ -25,7 +26,7 @@ class SplitKWorkspace:
 
     buffer: torch.Tensor          # u8, partial (max, sum-exp, out) slots + arrival counters
     output: torch.Tensor          # bf16 [B,Hq,128]; overwritten by every call
-    staging: torch.Tensor | None  # f32 [B,Hq,128], only when the cache dtype is not bf16
+    staging: torch.Tensor | None  # kept for the reference's field; the launch writes bf16 whatever the cache dtype
     block_n: int
     total_blocks: int
     num_query_heads: int
@@ -54,8 +55,7 @@ def _allocate(arenas: PackedArenas, num_query_heads: int, block_n: int, total_bl
     L.check(L.lib().r2k_decode_workspace_init(C.c_void_p(buffer.data_ptr()), C.c_size_t(nbytes),
                                               C.c_void_p(_stream_ptr(dev))), "r2k_decode_workspace_init")
     shape = (arenas.batch, num_query_heads, 128)
-    staging = None if arenas.dtype == torch.bfloat16 else torch.empty(shape, device=dev, dtype=torch.float32)
-    return SplitKWorkspace(buffer, torch.empty(shape, device=dev, dtype=torch.bfloat16), staging, int(block_n),
+    return SplitKWorkspace(buffer, torch.empty(shape, device=dev, dtype=torch.bfloat16), None, int(block_n),
                            int(total_blocks), int(num_query_heads))
 
 
@@ -123,6 +123,10 @@ class SplitKExecutor:
         self._ws_ptr, self._ws_size = workspace.buffer.data_ptr(), workspace.buffer.numel()
         self._qshape = (arenas.batch, self.num_query_heads, 128)
         self._host_staging, self._host_pair = None, None
+        # fp16 caches: the kernel's element type is fp16, the operator's output is bf16
+        self._flags = (L.FLAG_OUTPUT_HADAMARD if self.output_hadamard else 0) | (0 if arenas.dtype == torch.bfloat16 else L.FLAG_OUT_BF16)
+        self._step, self._batched = None, arenas.batch > 1
+        self._ring_capacity, self._static_tokens = arenas.recent_capacity, arenas.n_fp + arenas.n_i4
 
     @property
     def batched(self) -> bool:
@@ -187,23 +191,34 @@ class SplitKExecutor:
             ap.indices, ap.global_index, ap.logical_position = self._idx.data_ptr(), 0, 0
         return self._append_ref
 
+    def _make_step(self):
+        """The native per-step call: checks, argument block and launch (csrc/host_ext.cpp)."""
+        view = self.arenas.view()
+        self._view_obj, self._view_ref = view, C.byref(view)
+        self._step = host().Step(C.addressof(self._geom), C.addressof(view), self.workspace.buffer, self.workspace.output,
+                                 self.arenas.recent_k, self._flags)
+        return self._step
+
     def __call__(self, query: torch.Tensor, append=None) -> torch.Tensor:
-        query = self._check_query(query)
         a = self.arenas
-        if append is None and a.n_fp + a.n_i4 + a.i2_active + a.recent_len == 0:
-            raise ValueError("four-quadrant cache has no surviving tokens")
-        ap = self._make_append(append, query)
-        flags = L.FLAG_OUTPUT_HADAMARD if self.output_hadamard else 0
-        ws = self.workspace
-        if ws.staging is None:
-            self._launch(query, ap, ws.output.data_ptr(), flags)
-        else:
-            # fp16 caches: the kernel's element type is fp16, the operator's output is bf16
-            self._launch(query, ap, ws.staging.data_ptr(), flags | L.FLAG_OUT_F32)
-            ws.output.copy_(ws.staging)
-        if append is not None and self.batched:
+        step = self._step or self._make_step()
+        output = self.workspace.output
+        if append is None:
+            if a.recent_len == 0 and self._static_tokens + a.i2_active == 0:
+                raise ValueError("four-quadrant cache has no surviving tokens")
+            step.plain(query, a.i2_active)
+            return output
+        k, v, global_index, logical_position = append
+        if a.recent_len >= self._ring_capacity:
+            raise RuntimeError("prepared executor cannot fuse an append into a full Recent-FP pool")
+        if type(global_index) is int and type(logical_position) is int:
+            step.append(query, k, v, global_index, logical_position, a.i2_active)
+        else:   # per-request or device-resident indices
+            query = self._check_query(query)
+            self._launch(query, self._make_append(append, query), output.data_ptr(), self._flags)
+        if self._batched:
             a.recent_len += 1
-        return ws.output
+        return output
 
     def step_host(self, host_in: torch.Tensor, host_out: torch.Tensor, append_indices=None) -> torch.Tensor:
         """One decode step for a caller whose tensors live in host memory (r2k_decode_host): ``host_in`` is the

@@ -74,8 +74,6 @@ class SequenceShardedExecutor:
         self.state = torch.empty(shape, device=a.device, dtype=torch.float32)
         self.gathered = torch.empty((self.world * a.batch, local.num_query_heads, 130), device=a.device, dtype=torch.float32)
         self.output = torch.empty((a.batch, local.num_query_heads, 128), device=a.device, dtype=torch.bfloat16)
-        self._staging = None if a.dtype == torch.bfloat16 else torch.empty(self.output.shape, device=a.device,
-                                                                           dtype=torch.float32)
 
     def _open_exchange(self) -> None:
         """One exchange buffer per rank, created here and mapped into every other rank through its 64-byte
@@ -131,13 +129,8 @@ class SequenceShardedExecutor:
         else:
             states = self.state
         rows = a.batch * ex.num_query_heads
-        flags = L.FLAG_OUTPUT_HADAMARD if ex.output_hadamard else 0
-        out = self.output if self._staging is None else self._staging
-        if self._staging is not None:
-            flags |= L.FLAG_OUT_F32
+        flags = (L.FLAG_OUTPUT_HADAMARD if ex.output_hadamard else 0) | L.FLAG_OUT_BF16
         L.check(L.lib().r2k_merge_states(
             C.c_void_p(states.data_ptr()), self.world, C.c_int64(rows * 130), rows, dtype_code(a.dtype),
-            C.c_void_p(out.data_ptr()), C.c_uint32(flags), C.c_void_p(_stream_ptr(a.device))), "r2k_merge_states")
-        if self._staging is not None:
-            self.output.copy_(self._staging)
+            C.c_void_p(self.output.data_ptr()), C.c_uint32(flags), C.c_void_p(_stream_ptr(a.device))), "r2k_merge_states")
         return self.output
