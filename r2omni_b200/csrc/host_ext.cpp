@@ -237,6 +237,155 @@ py::tuple build_cache(const at::Tensor& key, const at::Tensor& value, const at::
   return py::make_tuple(std::move(t), n_fp, n_i4, n_i2);
 }
 
+// ---------------------------------------------------------------------------
+// rotation and Hadamard of a step's or a prefill's rows
+// ---------------------------------------------------------------------------
+void require(bool ok, const char* message) {
+  if (!ok) throw py::value_error(message);
+}
+void require_cuda(bool ok, const char* message) {
+  if (!ok) throw std::runtime_error(message);
+}
+bool row_type(at::ScalarType t) { return t == at::kBFloat16 || t == at::kHalf; }
+
+struct Rotary {
+  const void *cos, *sin;
+  int32_t type;
+  int64_t cos_strides[4], sin_strides[4];
+};
+Rotary rotary(const at::Tensor& cos, const at::Tensor& sin) {
+  require(cos.scalar_type() == sin.scalar_type() && (row_type(cos.scalar_type()) || cos.scalar_type() == at::kFloat),
+          "rotary tables must share one of bf16 / fp16 / fp32");
+  Rotary r;
+  r.cos = cos.data_ptr();
+  r.sin = sin.data_ptr();
+  r.type = cos.scalar_type() == at::kFloat ? 2 : dtype_code(cos.scalar_type());
+  for (int i = 0; i < 4; ++i) { r.cos_strides[i] = cos.stride(i); r.sin_strides[i] = sin.stride(i); }
+  return r;
+}
+void require_sections(const std::vector<int64_t>& s) {
+  require(s.size() == 3 && s[0] + s[1] + s[2] == 64, "Qwen mRoPE sections must contain three values summing to 64");
+}
+
+// triton_fwht_128 (r2omni/sspa/kernels/triton_qwen_mrope.py:325-346)
+at::Tensor fwht(const at::Tensor& tensor, const std::optional<at::Tensor>& output) {
+  require(tensor.dim() > 0 && tensor.size(-1) == 128 && tensor.is_floating_point(),
+          "fused FWHT requires a floating tensor with last dimension 128");
+  require_cuda(tensor.is_cuda(), "fused FWHT requires a CUDA tensor");
+  require(row_type(tensor.scalar_type()), "fused FWHT runs on bf16 / fp16 rows (the cache's element types)");
+  const c10::cuda::CUDAGuard guard(tensor.device());
+  const at::Tensor in = tensor.contiguous();
+  at::Tensor out;
+  if (output) {
+    out = *output;
+    require(out.sizes() == in.sizes() && out.device() == in.device() && out.scalar_type() == in.scalar_type(),
+            "fused FWHT output must match input shape, device, and dtype");
+    require(out.is_contiguous(), "fused FWHT output must be contiguous");
+  } else {
+    out = at::empty_like(in);
+  }
+  if (in.numel() > 0)
+    check(r2k_fwht128(in.data_ptr(), out.data_ptr(), dtype_code(in.scalar_type()), in.numel() / 128,
+                      at::cuda::getCurrentCUDAStream().stream()),
+          "r2k_fwht128");
+  return out;
+}
+
+// qwen_qk_mrope (r2omni/sspa/kernels/triton_qwen_mrope.py:214-322)
+std::pair<at::Tensor, at::Tensor> qk_mrope(const at::Tensor& query, const at::Tensor& key, const at::Tensor& cos, const at::Tensor& sin,
+                                           const std::vector<int64_t>& sections, const std::optional<std::vector<at::Tensor>>& output,
+                                           bool hadamard) {
+  require(query.dim() == 4 && key.dim() == 4, "Qwen fused mRoPE requires rank-4 Q/K");
+  const int64_t batch = query.size(0), tokens = query.size(2);
+  require(key.size(0) == batch, "Qwen fused mRoPE requires equal Q/K batch sizes");
+  require(tokens > 0 && key.size(2) == tokens, "Qwen fused mRoPE requires equal positive Q/K token counts");
+  require(query.size(3) == 128 && key.size(3) == 128, "Qwen fused mRoPE currently requires head_dim=128");
+  require(query.device() == key.device() && query.scalar_type() == key.scalar_type(), "Q/K device and dtype must match");
+  require(cos.device() == query.device() && sin.device() == query.device(), "Q/K and rotary tensors must share a device");
+  require(cos.dim() == 4 && cos.sizes() == sin.sizes() && cos.size(0) == 3, "Qwen fused mRoPE requires cos/sin [3,B,S,D]");
+  require(cos.size(1) == batch && cos.size(2) == tokens && cos.size(3) == 128, "Qwen fused mRoPE rotary positions must match Q/K tokens");
+  require_sections(sections);
+  require_cuda(query.is_cuda(), "fused Qwen mRoPE requires CUDA tensors");
+  require(row_type(query.scalar_type()), "fused Qwen mRoPE runs on bf16 / fp16 rows");
+  const Rotary rot = rotary(cos, sin);
+  const c10::cuda::CUDAGuard guard(query.device());
+  const at::Tensor q = query.contiguous(), k = key.contiguous();
+  at::Tensor qo, ko;
+  if (output) {
+    require(output->size() == 2 && (*output)[0].sizes() == q.sizes() && (*output)[1].sizes() == k.sizes(),
+            "fused Qwen mRoPE output shapes must match Q/K");
+    qo = (*output)[0];
+    ko = (*output)[1];
+    require(qo.device() == q.device() && ko.device() == q.device() && qo.scalar_type() == q.scalar_type() && ko.scalar_type() == q.scalar_type(),
+            "fused Qwen mRoPE outputs must match Q/K device and dtype");
+    require(qo.is_contiguous() && ko.is_contiguous(), "fused Qwen mRoPE outputs must be contiguous");
+  } else {
+    qo = at::empty_like(q);
+    ko = at::empty_like(k);
+  }
+  check(r2k_qk_mrope(q.data_ptr(), k.data_ptr(), qo.data_ptr(), ko.data_ptr(), dtype_code(q.scalar_type()), (int32_t)batch,
+                     (int32_t)q.size(1), (int32_t)k.size(1), (int32_t)tokens, rot.cos, rot.sin, rot.type, rot.cos_strides, rot.sin_strides,
+                     (int32_t)sections[0], (int32_t)sections[1], hadamard ? 1 : 0, at::cuda::getCurrentCUDAStream().stream()),
+        "r2k_qk_mrope");
+  return {qo, ko};
+}
+
+// A request's rows of `t` as one run of heads * 128 elements, requests `stride` elements apart; copies where there is no such view.
+struct Rows { at::Tensor t; int64_t heads, stride; };
+Rows request_rows(const at::Tensor& t, int64_t batch, const char* what) {
+  require_cuda(t.is_cuda(), "fused Qwen prologue requires CUDA tensors");
+  if (batch < 1 || t.size(0) != batch || t.numel() % (batch * 128) != 0)
+    throw py::value_error(std::string(what) + " rows do not match the batch");
+  Rows r{t, t.numel() / (batch * 128), t.numel() / batch};
+  if (t.is_contiguous()) return r;
+  if (t.dim() == 3 && t.size(1) == 1 && t.stride(2) == 1) {
+    r.stride = t.stride(0);
+  } else {
+    r.t = t.reshape({batch, r.heads * 128});
+    r.stride = r.t.stride(0);
+  }
+  if ((r.t.dim() == 2 && r.t.stride(1) != 1) || r.stride % 4 || reinterpret_cast<uintptr_t>(r.t.data_ptr()) % 8) {
+    r.t = r.t.contiguous();
+    r.stride = r.heads * 128;
+  }
+  return r;
+}
+
+// qwen_qkv_prologue: see its Python entry.
+std::vector<at::Tensor> qkv_prologue(const at::Tensor& query, const at::Tensor& key, const at::Tensor& value, const at::Tensor& cos,
+                                     const at::Tensor& sin, const std::vector<int64_t>& sections, bool key_hadamard, bool value_hadamard,
+                                     const std::optional<std::vector<at::Tensor>>& output) {
+  require(query.dim() > 0 && key.dim() > 0 && value.dim() > 0, "query rows do not match the batch");
+  const int64_t batch = query.size(0);
+  const Rows q = request_rows(query, batch, "query"), k = request_rows(key, batch, "key"), v = request_rows(value, batch, "value");
+  require(v.heads == k.heads, "key and value rows must have the same number of heads");
+  const at::ScalarType T = q.t.scalar_type();
+  require(row_type(T) && k.t.scalar_type() == T && v.t.scalar_type() == T, "fused Qwen prologue runs on bf16 / fp16 rows");
+  require(cos.dim() == 4 && cos.sizes() == sin.sizes() && cos.size(0) == 3 && cos.size(1) == batch && cos.size(2) == 1 && cos.size(3) == 128,
+          "Qwen fused prologue requires cos/sin [3,B,1,128]");
+  require(cos.device() == q.t.device() && sin.device() == q.t.device(), "Q/K and rotary tensors must share a device");
+  const Rotary rot = rotary(cos, sin);
+  require_sections(sections);
+  const c10::cuda::CUDAGuard guard(q.t.device());
+  std::vector<at::Tensor> out;
+  if (output) {
+    out = *output;
+    require(out.size() == 3, "fused Qwen prologue outputs must be contiguous [B,H,1,128] of the input type");
+    for (int i = 0; i < 3; ++i)
+      require(out[i].dim() == 4 && out[i].size(0) == batch && out[i].size(1) == (i == 0 ? q.heads : k.heads) && out[i].size(2) == 1 &&
+                  out[i].size(3) == 128 && out[i].scalar_type() == T && out[i].device() == q.t.device() && out[i].is_contiguous(),
+              "fused Qwen prologue outputs must be contiguous [B,H,1,128] of the input type");
+  } else {
+    for (int i = 0; i < 3; ++i) out.push_back(at::empty({batch, i == 0 ? q.heads : k.heads, 1, 128}, q.t.options()));
+  }
+  check(r2k_qkv_prologue(q.t.data_ptr(), q.stride, k.t.data_ptr(), k.stride, v.t.data_ptr(), v.stride, out[0].data_ptr(), out[1].data_ptr(),
+                         out[2].data_ptr(), dtype_code(T), (int32_t)batch, (int32_t)q.heads, (int32_t)k.heads, rot.cos, rot.sin, rot.type,
+                         rot.cos_strides, rot.sin_strides, (int32_t)sections[0], (int32_t)sections[1], key_hadamard ? 1 : 0,
+                         value_hadamard ? 1 : 0, at::cuda::getCurrentCUDAStream().stream()),
+        "r2k_qkv_prologue");
+  return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_r2k_host, m) {
@@ -245,4 +394,7 @@ PYBIND11_MODULE(_r2k_host, m) {
       .def("plain", &Step::plain)
       .def("append", &Step::append);
   m.def("build_cache", &build_cache);
+  m.def("fwht", &fwht);
+  m.def("qk_mrope", &qk_mrope);
+  m.def("qkv_prologue", &qkv_prologue);
 }

@@ -72,10 +72,6 @@ def dtype_code(dtype: torch.dtype) -> int:
     raise ValueError("the packed-KV path stores bfloat16 or float16 keys/values")
 
 
-def _ptr(t: torch.Tensor | None):
-    return None if t is None or t.numel() == 0 else C.c_void_p(t.data_ptr())
-
-
 # --------------------------------------------------------------------------- #
 # storage
 # --------------------------------------------------------------------------- #
