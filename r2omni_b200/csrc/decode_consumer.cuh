@@ -19,6 +19,32 @@ constexpr float k2m20 = 1.0f / 1048576.0f;
 constexpr uint32_t kMaskLo = 0x000F000Fu;  // nibble 0 of each half-word -> code * 2^-24 as fp16
 constexpr uint32_t kMaskHi = 0x00F000F0u;  // nibble 1 of each half-word -> code * 2^-20 as fp16
 
+// LOP3 takes one immediate: with two constants, (x & a) ^ b and (x & a) | b become two instructions each (64 more per
+// 32-token block of INT4 or INT2 values, a tenth of the block).  So the second constant comes in a register, read from
+// shared memory where the compiler cannot see through it.  Four 8 x 32768-token layers: 114.5 -> 107.3 us with INT4
+// values only, 120.4 -> 118.9 with INT2.
+template <uint32_t MASK>
+__device__ __forceinline__ uint32_t and_xor(uint32_t x, uint32_t c) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0x6A;\n" : "=r"(d) : "r"(x), "n"(MASK), "r"(c));
+  return d;
+}
+template <uint32_t MASK>
+__device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t c) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(d) : "r"(x), "n"(MASK), "r"(c));
+  return d;
+}
+constexpr uint32_t kFixLo = 0x00080008u, kFixHi = 0x00800080u;   // code ^ 8 of the low / high nibble pairs
+constexpr uint32_t kCrumbBase = 0x64006400u;                     // 1024 as half2
+// What a pool's loop keeps of them: INT4 values kFixLo four times (as an A operand of the MMA, too) and kFixHi;
+// INT2 values kCrumbBase.
+struct PoolConsts {
+  uint32_t f[4];
+  uint32_t x;
+};
+constexpr int kConstBytes = 32;   // the block in shared memory: four kFixLo, kFixHi, kCrumbBase
+
 // ---- shared-memory loads by 32-bit address (volatile: never hoisted above the stage's barrier wait) ----
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
@@ -145,64 +171,66 @@ struct LaneOffsets {
 // Scores of two 16-token tiles against INT4 keys.  Q' = q * scale is held as an exact two-term fp16 sum
 // (hi = RN(q*s), lo = fma(q, s, -hi)), so every product the tensor core sees is exact and the fp32
 // accumulation is the only rounding.  Codes minus zero points are fed as signed fp16 subnormals (AND, HSUB2).
+// The four 32-channel steps are the outer loop: Q' and the zero points of a step live for that step only (12 registers
+// instead of 48) and both tiles' four MMA chains run side by side.  Same sums in the same order as with the tiles
+// outermost; four 8 x 32768-token layers 128.5 -> 120.9 us, 16 x 4 heads x 65536 tokens 178.6 -> 167.7 us.
 __device__ __forceinline__ void qk_int4(uint32_t sb, const LaneOffsets& o, const uint32_t (&qh)[16], float alpha,
                                         float (&s)[2][4]) {
-  uint32_t qp[16], ql[16];  // paired (c0,c4) (c1,c5) (c2,c6) (c3,c7) per 8-channel word
+  uint32_t w[4][4];   // key words of row 16 j + 8 e (index 2 j + e), one per channel step
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const uint4 x = lds128(sb + o.k + 8 * r * 64);
+    w[r][0] = x.x; w[r][1] = x.y; w[r][2] = x.z; w[r][3] = x.w;
+  }
+  float lo[2][4], hi[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) lo[j][c] = hi[j][c] = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint4 w = lds128(sb + o.ks + 16 * i);
-    const uint32_t sp[4] = {__byte_perm(w.x, w.z, 0x5410), __byte_perm(w.x, w.z, 0x7632), __byte_perm(w.y, w.w, 0x5410),
-                            __byte_perm(w.y, w.w, 0x7632)};
+    const uint4 sc = lds128(sb + o.ks + 16 * i);
+    const uint2 z = lds64(sb + o.kz + 8 * i);
+    // paired (c0,c4) (c1,c5) (c2,c6) (c3,c7) of the 8-channel word
+    const uint32_t sp[4] = {__byte_perm(sc.x, sc.z, 0x5410), __byte_perm(sc.x, sc.z, 0x7632), __byte_perm(sc.y, sc.w, 0x5410),
+                            __byte_perm(sc.y, sc.w, 0x7632)};
+    uint32_t qp[4], ql[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      qp[4 * i + k] = hmul2_u32(qh[4 * i + k], sp[k]);
-      ql[4 * i + k] = hfma2_neg_u32(qh[4 * i + k], sp[k], qp[4 * i + k]);
+      qp[k] = hmul2_u32(qh[4 * i + k], sp[k]);
+      ql[k] = hfma2_neg_u32(qh[4 * i + k], sp[k], qp[k]);
     }
-  }
-  // Zero points as fp16 subnormal pairs in the two code domains: (z0,z4), (z2,z6) scaled 2^-24 for the low
-  // nibbles and (z1,z5), (z3,z7) scaled 2^-20 for the high ones.  code - zero is then one exact HSUB2 per
-  // register (subnormal arithmetic is exact on integers), and the tensor core sees signed integers.
-  uint32_t zl[8], zh[8];
-  {
-    const uint4 za = lds128(sb + o.kz), zb = lds128(sb + o.kz + 16);
-    const uint32_t z[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
+    // Zero points as fp16 subnormal pairs in the two code domains: (z0,z4), (z2,z6) scaled 2^-24 for the low
+    // nibbles and (z1,z5), (z3,z7) scaled 2^-20 for the high ones.  code - zero is then one exact HSUB2 per
+    // register (subnormal arithmetic is exact on integers), and the tensor core sees signed integers.
+    const uint32_t x = __byte_perm(z.x, z.y, 0x5410), y = __byte_perm(z.x, z.y, 0x7632);   // z0 z1 z4 z5, z2 z3 z6 z7
+    const uint32_t zl0 = x & 0x00FF00FFu, zh0 = (x >> 4) & 0x0FF00FF0u;
+    const uint32_t zl1 = y & 0x00FF00FFu, zh1 = (y >> 4) & 0x0FF00FF0u;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t x = __byte_perm(z[2 * i], z[2 * i + 1], 0x5410);  // z0 z1 z4 z5
-      const uint32_t y = __byte_perm(z[2 * i], z[2 * i + 1], 0x7632);  // z2 z3 z6 z7
-      zl[2 * i] = x & 0x00FF00FFu;     zh[2 * i] = (x >> 4) & 0x0FF00FF0u;
-      zl[2 * i + 1] = y & 0x00FF00FFu; zh[2 * i + 1] = (y >> 4) & 0x0FF00FF0u;
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t wa = w[2 * j][i], wb = w[2 * j + 1][i], a8 = wa >> 8, b8 = wb >> 8;
+      const uint32_t l0 = hsub2_u32(wa & kMaskLo, zl0), l1 = hsub2_u32(wb & kMaskLo, zl0);
+      const uint32_t l2 = hsub2_u32(a8 & kMaskLo, zl1), l3 = hsub2_u32(b8 & kMaskLo, zl1);
+      const uint32_t h0 = hsub2_u32(wa & kMaskHi, zh0), h1 = hsub2_u32(wb & kMaskHi, zh0);
+      const uint32_t h2 = hsub2_u32(a8 & kMaskHi, zh1), h3 = hsub2_u32(b8 & kMaskHi, zh1);
+      mma_f16(lo[j], l0, l1, l2, l3, qp[0], qp[2]);
+      mma_f16(hi[j], h0, h1, h2, h3, qp[1], qp[3]);
+      mma_f16(lo[j], l0, l1, l2, l3, ql[0], ql[2]);
+      mma_f16(hi[j], h0, h1, h2, h3, ql[1], ql[3]);
     }
   }
   const float f24 = k2p24 * alpha, f20 = k2p20 * alpha;
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const uint4 ka = lds128(sb + o.k + 16 * j * 64);
-    const uint4 kb = lds128(sb + o.k + (16 * j + 8) * 64);
-    const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb.x, kb.y, kb.z, kb.w};
-    float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t a8 = wa[i] >> 8, b8 = wb[i] >> 8;
-      const uint32_t l0 = hsub2_u32(wa[i] & kMaskLo, zl[2 * i]), l1 = hsub2_u32(wb[i] & kMaskLo, zl[2 * i]);
-      const uint32_t l2 = hsub2_u32(a8 & kMaskLo, zl[2 * i + 1]), l3 = hsub2_u32(b8 & kMaskLo, zl[2 * i + 1]);
-      const uint32_t h0 = hsub2_u32(wa[i] & kMaskHi, zh[2 * i]), h1 = hsub2_u32(wb[i] & kMaskHi, zh[2 * i]);
-      const uint32_t h2 = hsub2_u32(a8 & kMaskHi, zh[2 * i + 1]), h3 = hsub2_u32(b8 & kMaskHi, zh[2 * i + 1]);
-      mma_f16(lo, l0, l1, l2, l3, qp[4 * i + 0], qp[4 * i + 2]);
-      mma_f16(hi, h0, h1, h2, h3, qp[4 * i + 1], qp[4 * i + 3]);
-      mma_f16(lo, l0, l1, l2, l3, ql[4 * i + 0], ql[4 * i + 2]);
-      mma_f16(hi, h0, h1, h2, h3, ql[4 * i + 1], ql[4 * i + 3]);
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) s[j][c] = fmaf(lo[c], f24, hi[c] * f20);
-  }
+    for (int c = 0; c < 4; ++c) s[j][c] = fmaf(lo[j][c], f24, hi[j][c] * f20);
 }
 
 // O^T += V^T P^T for 16-token tile j of INT4 values: codes as fp16 subnormals (the two's-complement fix
 // code ^ 8 rides in the same LOP3 as the mask), per-token scale folded into P.
 template <bool PARTIAL>
-__device__ __forceinline__ void pv_int4(WarpState& st, uint32_t sb, const LaneOffsets& o, int j, float (&p)[4], int pg,
-                                        int lo, int hi) {
+__device__ __forceinline__ void pv_int4(WarpState& st, uint32_t sb, const LaneOffsets& o, int j, const PoolConsts& k,
+                                        float (&p)[4], int pg, int lo, int hi) {
   float sa = __uint_as_float(lds32(sb + o.m0 + 64 * j)), sc = __uint_as_float(lds32(sb + o.m0 + 64 * j + 32));
   if (PARTIAL) {
     if (16 * j + pg < lo || 16 * j + pg >= hi) sa = 0.f;
@@ -210,41 +238,43 @@ __device__ __forceinline__ void pv_int4(WarpState& st, uint32_t sb, const LaneOf
   }
   const uint32_t ha = pack_f16x2(p[0] * sa, p[1] * sa), hb = pack_f16x2(p[2] * sc, p[3] * sc);
   const uint32_t b0 = movmatrix_trans(ha), b1 = movmatrix_trans(hb);
-  mma_f16(st.corr, 0x00080008u, 0x00080008u, 0x00080008u, 0x00080008u, b0, b1);   // the offset the codes carry below
+  mma_f16(st.corr, k.f[0], k.f[1], k.f[2], k.f[3], b0, b1);   // the offset the codes carry below
   const uint2 w0 = lds64(sb + o.va + 1024 * j), w1 = lds64(sb + o.vb + 1024 * j);
   const uint2 w2 = lds64(sb + o.va + 1024 * j + 512), w3 = lds64(sb + o.vb + 1024 * j + 512);
-  constexpr uint32_t kFixLo = 0x00080008u, kFixHi = 0x00800080u;
 #pragma unroll
   for (int hf = 0; hf < 2; ++hf) {
     const uint32_t c0 = hf ? w0.y : w0.x, c1 = hf ? w1.y : w1.x, c2 = hf ? w2.y : w2.x, c3 = hf ? w3.y : w3.x;
     const uint32_t xa = __byte_perm(c0, c1, 0x5410), ya = __byte_perm(c0, c1, 0x7632);
     const uint32_t xb = __byte_perm(c2, c3, 0x5410), yb = __byte_perm(c2, c3, 0x7632);
     const uint32_t xa8 = xa >> 8, xb8 = xb >> 8, ya8 = ya >> 8, yb8 = yb >> 8;
-    mma_f16(st.o[4 * hf + 0], (xa & kMaskLo) ^ kFixLo, (xa & kMaskHi) ^ kFixHi, (xb & kMaskLo) ^ kFixLo, (xb & kMaskHi) ^ kFixHi, b0, b1);
-    mma_f16(st.o[4 * hf + 1], (xa8 & kMaskLo) ^ kFixLo, (xa8 & kMaskHi) ^ kFixHi, (xb8 & kMaskLo) ^ kFixLo, (xb8 & kMaskHi) ^ kFixHi, b0, b1);
-    mma_f16(st.o[4 * hf + 2], (ya & kMaskLo) ^ kFixLo, (ya & kMaskHi) ^ kFixHi, (yb & kMaskLo) ^ kFixLo, (yb & kMaskHi) ^ kFixHi, b0, b1);
-    mma_f16(st.o[4 * hf + 3], (ya8 & kMaskLo) ^ kFixLo, (ya8 & kMaskHi) ^ kFixHi, (yb8 & kMaskLo) ^ kFixLo, (yb8 & kMaskHi) ^ kFixHi, b0, b1);
+    mma_f16(st.o[4 * hf + 0], and_xor<kMaskLo>(xa, k.f[0]), and_xor<kMaskHi>(xa, k.x),
+            and_xor<kMaskLo>(xb, k.f[0]), and_xor<kMaskHi>(xb, k.x), b0, b1);
+    mma_f16(st.o[4 * hf + 1], and_xor<kMaskLo>(xa8, k.f[0]), and_xor<kMaskHi>(xa8, k.x),
+            and_xor<kMaskLo>(xb8, k.f[0]), and_xor<kMaskHi>(xb8, k.x), b0, b1);
+    mma_f16(st.o[4 * hf + 2], and_xor<kMaskLo>(ya, k.f[0]), and_xor<kMaskHi>(ya, k.x),
+            and_xor<kMaskLo>(yb, k.f[0]), and_xor<kMaskHi>(yb, k.x), b0, b1);
+    mma_f16(st.o[4 * hf + 3], and_xor<kMaskLo>(ya8, k.f[0]), and_xor<kMaskHi>(ya8, k.x),
+            and_xor<kMaskLo>(yb8, k.f[0]), and_xor<kMaskHi>(yb8, k.x), b0, b1);
   }
 }
 
 // (code - zero) * scale for the eight 2-bit fields of each half-word of x -> eight half2.
-__device__ __forceinline__ void dequant_crumbs(uint32_t x, const uint32_t (&zm)[5], const uint32_t (&sk)[5],
+__device__ __forceinline__ void dequant_crumbs(uint32_t x, uint32_t base, const uint32_t (&zm)[5], const uint32_t (&sk)[5],
                                                uint32_t (&v)[8]) {
-#pragma unroll
-  for (int i = 0; i < 5; ++i)
-    v[i] = hmul2_u32(hsub2_u32((x & (0x00030003u << (2 * i))) | 0x64006400u, zm[i]), sk[i]);
   const uint32_t y = x >> 10;
+  const uint32_t u[8] = {and_or<0x00030003u>(x, base), and_or<0x000C000Cu>(x, base), and_or<0x00300030u>(x, base),
+                         and_or<0x00C000C0u>(x, base), and_or<0x03000300u>(x, base), and_or<0x00030003u>(y, base),
+                         and_or<0x000C000Cu>(y, base), and_or<0x00300030u>(y, base)};
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
-    v[5 + i] = hmul2_u32(hsub2_u32((y & (0x00030003u << (2 * i))) | 0x64006400u, zm[i]), sk[i]);
+  for (int i = 0; i < 8; ++i) v[i] = hmul2_u32(hsub2_u32(u[i], zm[i % 5]), sk[i % 5]);
 }
 
 // O^T += V^T P^T for 16-token tile j of INT2 values, dequantised in registers ((code - zero) exactly, then one
 // fp16 multiply by the scale).  `step` = bytes between consecutive tokens of the scale array (2 * groups);
 // the zero array has half that pitch.  Token t1 sits one token after (t even) or before (t odd) token t0.
 template <bool PARTIAL>
-__device__ __forceinline__ void pv_int2(WarpState& st, uint32_t sb, const LaneOffsets& o, int j, float (&pr)[4], int t,
-                                        int step, int lo, int hi) {
+__device__ __forceinline__ void pv_int2(WarpState& st, uint32_t sb, const LaneOffsets& o, int j, const PoolConsts& k,
+                                        float (&pr)[4], int t, int step, int lo, int hi) {
   const uint32_t b0 = movmatrix_trans(pack_f16x2(pr[0], pr[1])), b1 = movmatrix_trans(pack_f16x2(pr[2], pr[3]));
   const int d1 = (t & 1) ? -step : step;   // scale offset of token t1 relative to token t0
   uint32_t w[4], sc[4], zp[4];
@@ -269,11 +299,11 @@ __device__ __forceinline__ void pv_int2(WarpState& st, uint32_t sb, const LaneOf
     uint32_t zm[5], sk[5];
     const uint32_t quarter[5] = {0x3C003C00u, 0x34003400u, 0x2C002C00u, 0x24002400u, 0x1C001C00u};  // 4^-i as half2
 #pragma unroll
-    for (int i = 0; i < 5; ++i) { zm[i] = 0x64006400u + (z2 << (2 * i)); sk[i] = i ? hmul2_u32(s2, quarter[i]) : s2; }
+    for (int i = 0; i < 5; ++i) { zm[i] = kCrumbBase + (z2 << (2 * i)); sk[i] = i ? hmul2_u32(s2, quarter[i]) : s2; }
     const uint32_t x = __byte_perm(w[2 * pr2], w[2 * pr2 + 1], 0x5410), y = __byte_perm(w[2 * pr2], w[2 * pr2 + 1], 0x7632);
     uint32_t lo8[8], hi8[8];
-    dequant_crumbs(x, zm, sk, lo8);
-    dequant_crumbs(y, zm, sk, hi8);
+    dequant_crumbs(x, k.x, zm, sk, lo8);
+    dequant_crumbs(y, k.x, zm, sk, hi8);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       if (pr2 == 0) { va[i] = lo8[i]; va[8 + i] = hi8[i]; } else { vb[i] = lo8[i]; vb[8 + i] = hi8[i]; }

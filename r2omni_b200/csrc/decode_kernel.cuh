@@ -464,7 +464,7 @@ __device__ __noinline__ void exchange_merge(const DecodeParams& p, uint32_t seq,
 // One warp's 32-token key block of a tile: scores, softmax update, value accumulation.
 template <int POOL, bool PARTIAL, bool BF16>
 __device__ __forceinline__ void consume_block(WarpState& st, uint32_t sb, const LaneOffsets& o, const uint32_t (&qh)[16],
-                                              float alpha, int t, int pg, int step, int lo, int hi) {
+                                              float alpha, const PoolConsts& pc, int t, int pg, int step, int lo, int hi) {
   float s[2][4];
   qk_int4(sb, o, qh, alpha, s);
   if (PARTIAL) { mask_scores(s[0], pg, lo, hi); mask_scores(s[1], 16 + pg, lo, hi); }
@@ -472,8 +472,8 @@ __device__ __forceinline__ void consume_block(WarpState& st, uint32_t sb, const 
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     if (POOL == 0) pv_fp<BF16, true>(st, sb, o.va, o.vb, j, s[j]);
-    else if (POOL == 1) pv_int4<PARTIAL>(st, sb, o, j, s[j], pg, lo, hi);
-    else pv_int2<PARTIAL>(st, sb, o, j, s[j], t, step, lo, hi);
+    else if (POOL == 1) pv_int4<PARTIAL>(st, sb, o, j, pc, s[j], pg, lo, hi);
+    else pv_int2<PARTIAL>(st, sb, o, j, pc, s[j], t, step, lo, hi);
   }
 }
 
@@ -484,7 +484,7 @@ __device__ __forceinline__ void consume_block(WarpState& st, uint32_t sb, const 
 template <int POOL, bool BF16>
 __device__ __forceinline__ void consume_pool(WarpState& st, const DecodeParams& p, int ua, int ub, int first, uint32_t stage0,
                                              uint64_t* full_bar, uint64_t* empty_bar, int& stage, uint32_t& phase, bool& alive,
-                                             const uint32_t (&qh)[16], int warp, int lane) {
+                                             const uint32_t (&qh)[16], uint32_t consts, int warp, int lane) {
   if (ua >= ub) return;
   const int g = lane >> 2, t = lane & 3, pg = pi_row(g);
   constexpr int kLen = POOL == 0 ? kTF : kTQ;
@@ -514,6 +514,14 @@ __device__ __forceinline__ void consume_pool(WarpState& st, const DecodeParams& 
     o.m0 = kOffV + kOffI2Scale + (slice + t0) * step + 2 * grp;
     o.m1 = kOffV + kOffI2Zero + (slice + t0) * (step >> 1) + grp;
   }
+  PoolConsts pc;
+  if (POOL == 1) {
+    const uint4 f = lds128(consts);
+    pc.f[0] = f.x; pc.f[1] = f.y; pc.f[2] = f.z; pc.f[3] = f.w;
+    pc.x = lds32(consts + 16);
+  } else if (POOL == 2) {
+    pc.x = lds32(consts + 20);
+  }
   set_units(st, POOL == 1 ? 1 : 0);
   const int parity = warp >= kHalf ? 1 : 0;
   int lo_edge = a0 - (w0 + (ua - first) * kLen) - slice;   // validity window of this warp's slice, slides with the tile
@@ -526,9 +534,9 @@ __device__ __forceinline__ void consume_pool(WarpState& st, const DecodeParams& 
     if (alive) {
       if (POOL != 0 || ((u & 1) == parity)) {
         const uint32_t sb = stage0 + stage * kStageBytes;
-        if (lo_edge <= 0 && hi_edge >= 32) consume_block<POOL, false, BF16>(st, sb, o, qh, p.qscale, t, pg, step, 0, 32);
+        if (lo_edge <= 0 && hi_edge >= 32) consume_block<POOL, false, BF16>(st, sb, o, qh, p.qscale, pc, t, pg, step, 0, 32);
         else if (min(hi_edge, 32) > max(lo_edge, 0))
-          consume_block<POOL, true, BF16>(st, sb, o, qh, p.qscale, t, pg, step, max(lo_edge, 0), min(hi_edge, 32));
+          consume_block<POOL, true, BF16>(st, sb, o, qh, p.qscale, pc, t, pg, step, max(lo_edge, 0), min(hi_edge, 32));
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty_bar[stage]);
@@ -547,7 +555,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
   float* scratch = reinterpret_cast<float*>(smem + kStages * kStageBytes);
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes + kScratchBytes);
   uint64_t* empty_bar = full_bar + kStages;
-  int* flags = reinterpret_cast<int*>(empty_bar + kStages);  // [0] last-arriver flag
+  uint32_t* const_block = reinterpret_cast<uint32_t*>(empty_bar + kStages);   // see PoolConsts
+  int* flags = reinterpret_cast<int*>(const_block) + kConstBytes / 4;  // [0] last-arriver flag
+  static_assert(kStages * 16 + kConstBytes + 8 <= 256, "control block");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cta = blockIdx.x;
@@ -558,6 +568,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], kNW); }
     mbar_fence_init();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) const_block[i] = kFixLo;
+    const_block[4] = kFixHi;
+    const_block[5] = kCrumbBase;
   }
   __syncthreads();
 
@@ -655,12 +669,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
       for (int k = 0; k < 4; ++k) qh[4 * i + k] = pack_f16x2(f[k], f[k + 4]);
     }
 
-    const uint32_t stage0 = smem_u32(stages);
-    consume_pool<0, BF16>(st, p, max(u0, 0), min(u1, p.nF), 0, stage0, full_bar, empty_bar, stage, phase, alive, qh, warp, lane);
+    const uint32_t stage0 = smem_u32(stages), consts = smem_u32(const_block);
+    consume_pool<0, BF16>(st, p, max(u0, 0), min(u1, p.nF), 0, stage0, full_bar, empty_bar, stage, phase, alive, qh, consts, warp, lane);
     consume_pool<1, BF16>(st, p, max(u0, p.nF), min(u1, p.nF + p.n4), p.nF, stage0, full_bar, empty_bar, stage, phase, alive,
-                          qh, warp, lane);
+                          qh, consts, warp, lane);
     consume_pool<2, BF16>(st, p, max(u0, p.nF + p.n4), min(u1, p.nF + p.n4 + p.n2), p.nF + p.n4, stage0, full_bar, empty_bar,
-                          stage, phase, alive, qh, warp, lane);
+                          stage, phase, alive, qh, consts, warp, lane);
     // residual window: kTR-token tiles, 16 tokens per warp; the lower half of the warps takes even tiles and the
     // upper half odd ones, so two tiles (the whole 128-token window) are in work at once
     set_units(st, 0);
