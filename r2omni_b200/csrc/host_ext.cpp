@@ -233,7 +233,7 @@ py::tuple build_cache(const at::Tensor& key, const at::Tensor& value, const at::
   b.i2_global = (int64_t*)ptr(15); b.i2_logical = (int64_t*)ptr(16);
   b.fp_global = (int64_t*)ptr(17); b.fp_logical = (int64_t*)ptr(18); b.i4_global = (int64_t*)ptr(19); b.i4_logical = (int64_t*)ptr(20);
   b.evicted_global = (int64_t*)ptr(21);
-  if (rows > 0) check(r2k_build_cache(&b, at::cuda::getCurrentCUDAStream().stream()), "r2k_build_cache");
+  check(r2k_build_cache(&b, at::cuda::getCurrentCUDAStream().stream()), "r2k_build_cache");   // without tokens, too: it clears the cache
   return py::make_tuple(std::move(t), n_fp, n_i4, n_i2);
 }
 
