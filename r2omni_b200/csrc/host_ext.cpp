@@ -63,6 +63,7 @@ struct Step {
 
   void launch(const at::Tensor& query, const R2KAppend* ap, int32_t n_i2) {
     const bool four = query.dim() == 4 && query.size(2) == 1;   // [B,Hq,1,128]
+    if (query.dim() == 4 && query.size(2) > 1) return launch(query.select(2, 0), ap, n_i2);   // its first token's rows
     if (!((query.dim() == 3 && query.size(2) == 128) || (four && query.size(3) == 128)) || query.size(0) != batch ||
         query.size(1) != heads || query.device() != device || query.scalar_type() != dtype || !query.is_contiguous())
       throw py::value_error("query does not match prepared split-K executor");

@@ -107,6 +107,15 @@ def test_a_cache_without_tokens_is_cleared():
         assert not a.k_packed.any() and not a.k_scale.any() and not a.i2_packed.any() and not a.recent_k.any()
 
 
+def test_query_of_several_tokens_decodes_its_first():
+    g = torch.Generator().manual_seed(5)
+    key, value = (torch.randn(1, 96, 128, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    cache = R.build_three_precision_cache(key, value, _plan([2, 2, 5], [32, 32, 32]), page_size=32)
+    ex = R.prepare_splitk_executor(cache, R.allocate_splitk_workspace(cache, num_query_heads=1))
+    query = torch.randn(1, 1, 3, 128, generator=g).to(torch.bfloat16).cuda()
+    assert torch.equal(ex(query).clone(), ex(query[:, :, 0]))
+
+
 @pytest.mark.parametrize("sections", [(16, 24, 24), (15, 26, 23)])   # the second ends an axis inside an eight-channel word
 @pytest.mark.parametrize("shift", [0, 4])                            # rows on 16-byte boundaries and 8 bytes off them
 @pytest.mark.parametrize("batch,hq,hkv,tokens", [(1, 3, 1, 5), (3, 16, 2, 67), (1, 2, 1, 4099)])
