@@ -41,15 +41,15 @@ struct Step {
   const R2KCacheView* view;
   void* workspace;
   size_t workspace_bytes;
-  at::Tensor output;
+  at::Tensor buffer, output;
   at::ScalarType dtype;
   c10::Device device;
   uint32_t flags;
   int64_t batch, heads, kv_numel;
 
-  Step(uintptr_t geom_, uintptr_t view_, const at::Tensor& buffer, const at::Tensor& output_, const at::Tensor& like, uint32_t flags_)
-      : geom(reinterpret_cast<R2KGeom*>(geom_)), view(reinterpret_cast<const R2KCacheView*>(view_)), workspace(buffer.data_ptr()),
-        workspace_bytes((size_t)buffer.numel()), output(output_), dtype(like.scalar_type()), device(like.device()), flags(flags_),
+  Step(uintptr_t geom_, uintptr_t view_, const at::Tensor& buffer_, const at::Tensor& output_, const at::Tensor& like, uint32_t flags_)
+      : geom(reinterpret_cast<R2KGeom*>(geom_)), view(reinterpret_cast<const R2KCacheView*>(view_)), workspace(buffer_.data_ptr()),
+        workspace_bytes((size_t)buffer_.numel()), buffer(buffer_), output(output_), dtype(like.scalar_type()), device(like.device()), flags(flags_),
         batch(geom->batch), heads(geom->num_q_heads), kv_numel((int64_t)geom->batch * geom->num_kv_heads * 128) {}
 
   // ap filled from (k, v); the indices are the caller's business

@@ -201,7 +201,9 @@ class SplitKExecutor:
 
     def __call__(self, query: torch.Tensor, append=None) -> torch.Tensor:
         a = self.arenas
-        step = self._step or self._make_step()
+        step = self._step
+        if step is None or a._view is not self._view_obj:
+            step = self._make_step()
         output = self.workspace.output
         if append is None:
             if a.recent_len == 0 and self._static_tokens + a.i2_active == 0:
