@@ -48,6 +48,8 @@ constexpr int kRowFloats = 132;                  // (max, sum, pad, pad, out[128
 constexpr int kSlotFloats = 8 * kRowFloats;      // one partial: 8 heads of a KV group
 constexpr int kScratchBytes = kNW * kSlotFloats * 4;
 constexpr int kSmemBytes = kStages * kStageBytes + kScratchBytes + 256;
+constexpr int kCluster = 8;                      // CTAs of a head that merge through distributed shared memory
+constexpr int kClusterSmemBytes = kSmemBytes + kSlotFloats * 4;
 
 // Partials of a (request, kv head) are merged in groups of kMergeGroup by each group's last-arriving CTA, then the
 // group results by the head's last arriver.  A group is one batch of loads for the merging CTA (merge_rows), so
@@ -97,6 +99,7 @@ struct DecodeParams {
   uint32_t xseq, xflags_off;
   uint32_t xnap;                  // nanoseconds the cross-rank wait sleeps between two polls
   float* xbuf[R2K_MAX_RANKS];
+  int cluster;                    // host only: != 0 for kCluster CTAs per (request, kv head), launched as one cluster
   alignas(64) CUtensorMap fp_map;
 };
 

@@ -24,6 +24,7 @@
 //   * partial states go to a small workspace; the last CTA to finish a group of nine partials merges them, the
 //     last group of a (request, kv head) merges the group results, writes the output, applies the optional
 //     Hadamard epilogue and the fused append.
+//   * a few short heads take one cluster of eight CTAs each and merge through distributed shared memory.
 //   * the residual window is read in 64-token tiles, 16 tokens per warp, two tiles in work at once.
 //
 // Every wait is bounded: a wait that gives up records R2K_ERR_DEVICE_TIMEOUT in
@@ -270,11 +271,69 @@ __device__ __forceinline__ void merge_rows(const float* base, int count, int own
   }
 }
 
+// The same for the kCluster partials of a cluster's CTAs, read out of their shared memory (`slot`: this CTA's own).
+__device__ __forceinline__ void merge_cluster_rows(const float* slot, int hh, int sub, float& mx, float& lsum, float (&acc)[8]) {
+  float4 ml[kCluster], va[kCluster], vb[kCluster];
+  const uint32_t row = smem_u32(slot + hh * kRowFloats);
+#pragma unroll
+  for (int k = 0; k < kCluster; ++k) {
+    const uint32_t a = cluster_map(row, (uint32_t)k);
+    ml[k] = ld_cluster_f4(a);
+    va[k] = ld_cluster_f4(a + 16 + 32 * sub);
+    vb[k] = ld_cluster_f4(a + 32 + 32 * sub);
+  }
+  mx = -INFINITY;
+#pragma unroll
+  for (int k = 0; k < kCluster; ++k) mx = fmaxf(mx, ml[k].x);
+  lsum = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+#pragma unroll
+  for (int k = 0; k < kCluster; ++k) {
+    const float w = ml[k].x != -INFINITY ? ex2_approx(ml[k].x - mx) : 0.f;
+    acc[0] += w * va[k].x; acc[1] += w * va[k].y; acc[2] += w * va[k].z; acc[3] += w * va[k].w;
+    acc[4] += w * vb[k].x; acc[5] += w * vb[k].y; acc[6] += w * vb[k].z; acc[7] += w * vb[k].w;
+    lsum += w * ml[k].y;
+  }
+}
+
 __device__ __forceinline__ void store_row(float* slot, int hh, int sub, float mx, float lsum, const float (&acc)[8]) {
   float* orow = slot + hh * kRowFloats;
   __stcg(reinterpret_cast<float4*>(orow + 4 + 8 * sub), make_float4(acc[0], acc[1], acc[2], acc[3]));
   __stcg(reinterpret_cast<float4*>(orow + 8 + 8 * sub), make_float4(acc[4], acc[5], acc[6], acc[7]));
   if (sub == 0) __stcg(reinterpret_cast<float2*>(orow), make_float2(mx, lsum));
+}
+
+// Every CTA of (b, h) has arrived, so none of them reads recent_len[b] any more.  One thread outside the merge workers
+// counts the head in; the last head of the request moves the ring metadata; another warp writes the new rows.
+static_assert(kNW >= 6, "warps 4 and 5 carry the request counter and the appended rows");
+__device__ __forceinline__ void commit_append(const DecodeParams& p, int b, int h, int rlen0) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool has_append = p.app_k != nullptr;
+  if (threadIdx.x == 128) {
+    __threadfence();
+    const int done = atomicAdd(&p.req_counter[b], 1);
+    if (done == p.g.num_kv_heads - 1) {
+      p.req_counter[b] = 0;
+      if (has_append) {
+        const int64_t gi = p.app_idx ? p.app_idx[2 * b] : p.app_global;
+        const int64_t lp = p.app_idx ? p.app_idx[2 * b + 1] : p.app_logical;
+        *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_global + (size_t)b * p.v.recent_global_bstride + 8 * (size_t)rlen0) = gi;
+        *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_logical + (size_t)b * p.v.recent_logical_bstride + 8 * (size_t)rlen0) = lp;
+        *reinterpret_cast<int*>((uint8_t*)p.v.recent_len + (size_t)b * p.v.recent_len_bstride) = rlen0 + 1;
+        *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_page_lengths + (size_t)b * p.v.recent_page_lengths_bstride +
+                                    8 * (size_t)(rlen0 / p.g.page_size)) = rlen0 % p.g.page_size + 1;
+      }
+    }
+  }
+  if (has_append && warp == 5) {  // ring row rlen0 of head h
+    const size_t src = ((size_t)b * p.g.num_kv_heads + h) * 256 + 8 * lane;
+    const size_t dst = ((size_t)h * p.g.recent_capacity + rlen0) * 256 + 8 * lane;
+    *reinterpret_cast<uint2*>((uint8_t*)p.v.recent_k + (size_t)b * p.v.recent_k_bstride + dst) =
+        __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_k + src));
+    *reinterpret_cast<uint2*>((uint8_t*)p.v.recent_v + (size_t)b * p.v.recent_v_bstride + dst) =
+        __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_v + src));
+  }
 }
 
 // Normalise (or emit the raw state), optional Hadamard, store.  16 threads per head, 8 dims each.
@@ -548,12 +607,15 @@ __device__ __forceinline__ void consume_pool(WarpState& st, const DecodeParams& 
 // ---------------------------------------------------------------------------
 // kernel
 // ---------------------------------------------------------------------------
-template <bool BF16>
+// CLUSTER: launched in clusters of kCluster CTAs, one (request, kv head) each (a template parameter: the branch alone
+// cost the other launches 1 %).
+template <bool BF16, bool CLUSTER>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __grid_constant__ DecodeParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* stages = smem;
   float* scratch = reinterpret_cast<float*>(smem + kStages * kStageBytes);
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes + kScratchBytes);
+  float* cluster_slot = scratch + kNW * kSlotFloats;   // this CTA's partial, where the cluster's other CTAs read it
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(cluster_slot + (CLUSTER ? kSlotFloats : 0));
   uint64_t* empty_bar = full_bar + kStages;
   uint32_t* const_block = reinterpret_cast<uint32_t*>(empty_bar + kStages);   // see PoolConsts
   int* flags = reinterpret_cast<int*>(const_block) + kConstBytes / 4;  // [0] last-arriver flag
@@ -738,7 +800,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
     }
     named_bar_sync(1, kConsumers);
     float* slot = p.partials + ((size_t)bh * p.parts_cap + (cta - part0)) * kSlotFloats;
-    static_assert(kNW >= 6, "warps 4 and 5 carry the request counter and the appended rows");
     const bool worker = threadIdx.x < 128;   // warps 0-3 carry the merge protocol; the others only meet the barriers
     float own_m = -INFINITY, own_l = 0.f, own_acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // this CTA's partial
     if (worker) {
@@ -758,13 +819,37 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
         a1.x += wgt * v1.x; a1.y += wgt * v1.y; a1.z += wgt * v1.z; a1.w += wgt * v1.w;
         lsum += wgt * row[1];
       }
-      float* orow = slot + hh * kRowFloats;
-      __stcg(reinterpret_cast<float4*>(orow + 4 + 8 * sub), a0);
-      __stcg(reinterpret_cast<float4*>(orow + 8 + 8 * sub), a1);
-      if (sub == 0) __stcg(reinterpret_cast<float2*>(orow), make_float2(mx, lsum));
       own_m = mx; own_l = lsum;
       own_acc[0] = a0.x; own_acc[1] = a0.y; own_acc[2] = a0.z; own_acc[3] = a0.w;
       own_acc[4] = a1.x; own_acc[5] = a1.y; own_acc[6] = a1.z; own_acc[7] = a1.w;
+      if (CLUSTER) {
+        float* orow = cluster_slot + hh * kRowFloats;
+        *reinterpret_cast<float4*>(orow + 4 + 8 * sub) = a0;
+        *reinterpret_cast<float4*>(orow + 8 + 8 * sub) = a1;
+        if (sub == 0) *reinterpret_cast<float4*>(orow) = make_float4(mx, lsum, 0.f, 0.f);
+      } else {
+        store_row(slot, hh, sub, own_m, own_l, own_acc);
+      }
+    }
+    if (CLUSTER) {
+      // ---- one exact merge through distributed shared memory: the CTA of rank r merges head r of the group ----
+      // Two cluster barriers and one round of remote loads where the path below pays a store, a fence, a ticket and a
+      // round of loads through L2.  A cluster's CTAs hold one (request, kv head) each, so all of them come here once.
+      cluster_arrive();
+      cluster_wait();
+      const int rank = (int)cluster_rank();
+      if (warp == 0) {   // both halves of the warp do the same; the lower one stores
+        const int sub = lane & 15;
+        float mx, lsum, acc[8];
+        merge_cluster_rows(cluster_slot, rank, sub, mx, lsum, acc);
+        write_output<BF16>(p, (size_t)b * p.g.num_q_heads + h * p.gqa + rank, rank < p.gqa && lane < 16, sub, mx, lsum, acc);
+      } else if (rank == 0) {
+        commit_append(p, b, h, rlen0);
+      }
+      __syncwarp();
+      cluster_arrive();   // nobody leaves while its partial may still be read
+      cluster_wait();
+      return;
     }
     // ---- two-level exact merge: groups of kMergeGroup partials, then the group results ----
     // Release pattern: the CTA barrier orders every thread's partial stores before thread 0's fence, whose
@@ -811,34 +896,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
       }
     }
     if (last) {
-      // ---- last arriver of (b, h): epilogue and fused append ----
-      // Every CTA of this head has arrived, so none of them reads recent_len[b] any more.  One thread outside
-      // the merge workers counts the head in; the last head of the request moves the ring metadata.  This runs
-      // beside the merge below, not after it.
-      if (threadIdx.x == 128) {
-        __threadfence();
-        const int done = atomicAdd(&p.req_counter[b], 1);
-        if (done == p.g.num_kv_heads - 1) {
-          p.req_counter[b] = 0;
-          if (has_append) {
-            const int64_t gi = p.app_idx ? p.app_idx[2 * b] : p.app_global;
-            const int64_t lp = p.app_idx ? p.app_idx[2 * b + 1] : p.app_logical;
-            *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_global + (size_t)b * p.v.recent_global_bstride + 8 * (size_t)rlen0) = gi;
-            *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_logical + (size_t)b * p.v.recent_logical_bstride + 8 * (size_t)rlen0) = lp;
-            *reinterpret_cast<int*>((uint8_t*)p.v.recent_len + (size_t)b * p.v.recent_len_bstride) = rlen0 + 1;
-            *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_page_lengths + (size_t)b * p.v.recent_page_lengths_bstride +
-                                        8 * (size_t)(rlen0 / p.g.page_size)) = rlen0 % p.g.page_size + 1;
-          }
-        }
-      }
-      if (has_append && warp == 5) {  // ring row rlen0 of head h
-        const size_t src = ((size_t)b * p.g.num_kv_heads + h) * 256 + 8 * lane;
-        const size_t dst = ((size_t)h * p.g.recent_capacity + rlen0) * 256 + 8 * lane;
-        *reinterpret_cast<uint2*>((uint8_t*)p.v.recent_k + (size_t)b * p.v.recent_k_bstride + dst) =
-            __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_k + src));
-        *reinterpret_cast<uint2*>((uint8_t*)p.v.recent_v + (size_t)b * p.v.recent_v_bstride + dst) =
-            __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_v + src));
-      }
+      // ---- last arriver of (b, h): epilogue and fused append, beside the merge below ----
+      commit_append(p, b, h, rlen0);
       const size_t orow = (size_t)b * p.g.num_q_heads + h * p.gqa + hh;
       if (p.xw > 1) exchange_merge(p, xstep, orow, hh, worker, sub, scratch, mx, lsum, acc);
       if (worker) write_output<BF16>(p, orow, hh < p.gqa, sub, mx, lsum, acc);

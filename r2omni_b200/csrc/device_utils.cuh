@@ -184,6 +184,27 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Thread-block clusters.  An arrival releases, a wait acquires: what any thread of the cluster wrote to its shared memory
+// before it arrived can be read by all of them behind the wait.  Threads that have exited do not count.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+// Address of `a` (this CTA's shared memory) in the CTA of rank `rank`, and a 16-byte load from there.
+__device__ __forceinline__ uint32_t cluster_map(uint32_t a, uint32_t rank) {
+  uint32_t d;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(d) : "r"(a), "r"(rank));
+  return d;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+
 // Programmatic dependent launch.  launch_dependents lets the next kernel of the stream (when it was launched with
 // programmatic stream serialization) start its CTAs on SMs this grid has left; grid_dependency_wait blocks until
 // every kernel this grid depends on has completed and its writes are visible.  Both are no-ops otherwise.

@@ -18,6 +18,7 @@ std::atomic<uint64_t> g_launches{0};
 
 struct DeviceInfo {
   int sms = 0;
+  int clusters = 0;   // decode clusters that fit on the device at once
   bool ready = false;
   bool pdl = true;   // R2K_DISABLE_PDL=1 in the environment turns programmatic dependent launch off (debugging)
 };
@@ -34,12 +35,25 @@ int device_info(DeviceInfo** out) {
   if (!d.ready) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return R2K_ERR_CUDA;
-    if (cudaFuncSetAttribute(decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
+    auto prepare = [](auto kernel, int smem) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
+      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      return true;
+    };
+    if (!prepare(decode_kernel<true, false>, kSmemBytes) || !prepare(decode_kernel<false, false>, kSmemBytes) ||
+        !prepare(decode_kernel<true, true>, kClusterSmemBytes) || !prepare(decode_kernel<false, true>, kClusterSmemBytes))
       return R2K_ERR_CUDA;
-    cudaFuncSetAttribute(decode_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(decode_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     d.sms = sms;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {(unsigned)kCluster, 1u, 1u};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)kCluster);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kClusterSmemBytes;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&d.clusters, decode_kernel<true, true>, &cfg) != cudaSuccess) { cudaGetLastError(); d.clusters = 0; }
     const char* off = std::getenv("R2K_DISABLE_PDL");
     d.pdl = !(off != nullptr && off[0] == '1');
     d.ready = true;
@@ -141,14 +155,25 @@ int derive(const R2KGeom* g, DecodeParams* p) {
     const int rounded = p->grid / p->bh_total * p->bh_total;
     if (rounded * 20 >= p->grid * 19) p->grid = rounded;
   }
+  double head_ns = 0.0;
+  for (int k = 0; k < 4; ++k) head_ns += (double)cnt[k] * ns[k];
+  const double per_head = (double)p->grid / p->bh_total;
+  // Few heads with few tiles: kCluster CTAs per (request, kv head), one cluster, merge through distributed shared
+  // memory instead of the workspace, which takes 1.3 us off a launch (36 launches of 701 tokens x 2 heads: 300 -> 252 us;
+  // eight of 700 x 8 heads: 74.6 -> 67.5, of 4500 x 8: 97.4 -> 91.8).  Two lines bound it.  Time: fewer CTAs stream longer; eight launches of one
+  // request x 2 heads take 90.2 us without and 76.0 with clusters at 5000 tokens (4.3 us of tile weight more per CTA),
+  // 89.2 and 94.9 at 6500 (6.1 us).  Room: at most two thirds of the clusters that fit, so that some of the next launch's
+  // come in and fetch while this one finishes; 12 heads of 3000 tokens took 88.6 us without and 98.0 with clusters.
+  if (p->grid > p->bh_total && 3 * p->bh_total <= 2 * dev->clusters && kCluster * p->bh_total <= cap && p->c_bh >= (uint32_t)kCluster &&
+      head_ns / kCluster - head_ns / per_head < 5000.0) {
+    p->grid = kCluster * p->bh_total;
+    p->cluster = 1;
+  }
   // More than kMergeGroup CTAs on a (request, kv head) pay a second merge level (a store, a ticket and one more
   // round of loads: ~2.6 us).  A head with so few tiles that kMergeGroup CTAs stream them in less extra time than
   // that gets kMergeGroup CTAs: measured 11.3 -> 10.0 us per launch for one request x 2 kv heads x 4096 tokens
   // (18 -> 9 CTAs per head).  The tile weights include fixed costs (about 1.5x the streaming time), hence 3 us.
   if (p->grid > kMergeGroup * p->bh_total) {
-    double head_ns = 0.0;
-    for (int k = 0; k < 4; ++k) head_ns += (double)cnt[k] * ns[k];
-    const double per_head = (double)p->grid / p->bh_total;
     if (head_ns / kMergeGroup - head_ns / per_head < 3000.0) p->grid = kMergeGroup * p->bh_total;
   }
   if ((int64_t)p->grid * p->bh_total >= (int64_t)1 << 31) return R2K_ERR_GEOMETRY;
@@ -430,6 +455,7 @@ static int decode_impl(const R2KGeom* geom, const R2KCacheView* view, const void
       p.xnap = nap > 1000000u ? 1000000u : (uint32_t)nap;
     }
     p.xflags_off = (uint32_t)exchange_states_bytes(geom, ex->world);
+    p.cluster = 0;   // the fused cross-rank merge runs on the head's last arriver
   }
 
   DeviceInfo* dev;
@@ -439,7 +465,7 @@ static int decode_impl(const R2KGeom* geom, const R2KCacheView* view, const void
   // Programmatic stream serialization: when the previous kernel of the stream signals early (a decode launch
   // does), this grid's CTAs may start on free SMs and prefetch pool tiles; the kernel itself waits for the
   // previous kernel's completion before it reads anything that kernel can have written.
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = dev->pdl ? 1 : 0;
   cudaLaunchConfig_t cfg = {};
@@ -449,8 +475,16 @@ static int decode_impl(const R2KGeom* geom, const R2KCacheView* view, const void
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t err = geom->dtype == R2K_DTYPE_BF16 ? cudaLaunchKernelEx(&cfg, decode_kernel<true>, p)
-                                                        : cudaLaunchKernelEx(&cfg, decode_kernel<false>, p);
+  if (p.cluster) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim = {(unsigned)kCluster, 1u, 1u};
+    cfg.numAttrs = 2;
+    cfg.dynamicSmemBytes = kClusterSmemBytes;
+  }
+  const bool bf16 = geom->dtype == R2K_DTYPE_BF16;
+  const auto kernel = p.cluster ? (bf16 ? decode_kernel<true, true> : decode_kernel<false, true>)
+                                : (bf16 ? decode_kernel<true, false> : decode_kernel<false, false>);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, p);
   ++g_launches;
   return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
 }

@@ -1,0 +1,62 @@
+"""The decode launch of small caches (few tiles per head, few heads: one cluster of eight CTAs per head, merged through
+distributed shared memory) against the oracle and against the general launch, which a grid limit brings back."""
+import pytest
+import torch
+
+import r2omni_b200 as R
+from gpu_helpers import assert_close, make_executor
+from oracle import sspa_oracle as O
+from test_gpu_decode import both_caches, seeded_classes
+
+pytestmark = pytest.mark.gpu
+
+
+# from one tile in all (most of a cluster's CTAs idle) past the longest cache that takes clusters; one to eight heads;
+# every group width at its ends
+@pytest.mark.parametrize("hq,hkv,pages,page", [(16, 2, 1, 16), (16, 2, 3, 32), (7, 1, 11, 64), (2, 2, 20, 32), (28, 4, 16, 64),
+                                               (4, 4, 37, 16), (16, 2, 64, 64), (16, 2, 100, 64), (5, 5, 16, 64), (8, 8, 12, 64)])
+@pytest.mark.parametrize("dtype,hadamard", [(torch.bfloat16, False), (torch.float16, True)])
+def test_small_caches_through_a_flush(hq, hkv, pages, page, dtype, hadamard, monkeypatch):
+    tokens = pages * page
+    ocache, gcache, new_k, new_v, queries = both_caches(31 + pages, hq=hq, hkv=hkv, tokens=tokens, page=page,
+                                                        classes=seeded_classes(pages, pages), appends=131, dtype=dtype,
+                                                        append_capacity=256)
+    ex = make_executor(gcache, hq, output_hadamard=hadamard)
+    stats = R.DynamicCacheStats()
+    k, v, q = new_k.cuda(), new_v.cuda(), queries[0].cuda()
+    for i in range(131):
+        O.append_token(ocache, new_k[i], new_v[i], tokens + i, tokens + i)
+        ring = gcache.recent_fp_pool
+        if ring.active_length == ring.capacity:
+            R.flush_recent(gcache.arenas, stats)
+        ex(q, append=(k[i].unsqueeze(0).contiguous(), v[i].unsqueeze(0).contiguous(), tokens + i, tokens + i))
+        ring.active_length += 1
+        if i in (0, 63, 64, 127, 128, 130) and not hadamard:
+            assert_close(ex.decode_f32(q), O.decode_fp32(queries[0].float(), ocache), f"step {i}")
+    assert stats.flushed_tokens == 128 and int(gcache.arenas.recent_len_device) == ocache.recent_len
+    assert torch.equal(gcache.arenas.recent_global[0, :3].cpu(), torch.arange(tokens + 128, tokens + 131))
+    here = ex(queries[1].cuda()).float().clone()
+    monkeypatch.setenv("R2K_GRID_CAP", str(7 * hkv))   # below eight CTAs per head: the general launch
+    assert_close(here, ex(queries[1].cuda()).float(), "cluster against general launch")
+    assert ex.device_status() == 0
+
+
+def test_replayed_from_a_graph():
+    pages = 12
+    ocache, gcache, _, _, queries = both_caches(3, hq=16, hkv=2, tokens=pages * 64, page=64, classes=seeded_classes(pages, 3), appends=1)
+    ex = make_executor(gcache, 16)
+    q = queries[0].cuda()
+    eager = ex(q).clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        ex(q)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(4):
+            out = ex(q)
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)
