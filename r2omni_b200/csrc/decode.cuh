@@ -26,13 +26,15 @@ constexpr int kOffV = 0;
 // bf16-value tiles are stored as two half boxes (channels 0-63, 64-127) of kTF rows x 128 bytes; inside every
 // row the 16-byte chunks are XOR-swizzled by (row & 7) -- the layout of a 128-byte-swizzled tensor copy.
 constexpr int kFpHalfBytes = kTF * 128;
+// Per-token metadata arrives with the 16-byte granules it lies in and starts up to 15 bytes into its region, which is
+// why these regions are 16 bytes longer than their rows (meta_shift in decode_kernel.cuh).
 constexpr int kOffI4Scale = kTQ * 64;            // f32 per token after the nibble rows
 constexpr int kOffI2Scale = kTQ * 32;            // f16 x groups per token after the crumb rows
-constexpr int kOffI2Zero = kOffI2Scale + kTQ * 8;
+constexpr int kOffI2Zero = kOffI2Scale + kTQ * 8 + 16;
 constexpr int kOffRecentV = kTR * 256;           // residual tile: K rows then V rows
 constexpr int kVBytesFp = kTF * 256;
-constexpr int kVBytesPacked = kTQ * 68;
-static_assert(kOffI2Zero + kTQ * 4 <= kVBytesPacked && kOffI4Scale + kTQ * 4 <= kVBytesPacked, "value region");
+constexpr int kVBytesPacked = kTQ * 68 + 128;
+static_assert(kOffI2Zero + kTQ * 4 + 16 <= kVBytesPacked && kOffI4Scale + kTQ * 4 + 16 <= kVBytesPacked, "value region");
 __host__ __device__ constexpr int tile_tokens(int pool) { return pool == 0 ? kTF : kTQ; }
 __host__ __device__ constexpr int off_k(int pool) { return pool == 0 ? kVBytesFp : kVBytesPacked; }       // key nibble rows
 __host__ __device__ constexpr int off_ks(int pool) { return off_k(pool) + tile_tokens(pool) * 64; }          // key scales

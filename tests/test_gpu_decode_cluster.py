@@ -60,3 +60,31 @@ def test_replayed_from_a_graph():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, eager)
+
+
+@pytest.mark.parametrize("tail", [1, 2, 3, 13])   # INT4 pool lengths off multiples of four: scales of the later heads unaligned
+@pytest.mark.parametrize("pages,cap", [(9, None), (70, None), (70, 4)])
+def test_heads_behind_an_odd_int4_pool(tail, pages, cap, monkeypatch):
+    page, heads = 16, 4
+    lengths = torch.full((pages + 1,), page)
+    lengths[-1] = tail
+    classes = torch.cat((seeded_classes(pages, pages), torch.tensor([2])))
+    total = int(lengths.sum())
+    g = torch.Generator().manual_seed(total)
+    key, value = (torch.randn(heads, total, 128, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    query = torch.randn(1, heads * 7, 128, generator=g).to(torch.bfloat16).cuda()
+    sel = lambda c: (classes == c).nonzero().flatten()  # noqa: E731
+
+    def decode(rows, q):
+        plan = R.LayerCompressionPlan(
+            layer_id=0, fp_pages=sel(1), int4_pages=sel(2), int2_pages=sel(5), evicted_pages=sel(0),
+            protected_pages=torch.empty(0, dtype=torch.long), recent_fp_capacity=128, logical_positions=torch.arange(total),
+            global_token_indices=torch.arange(total), page_offsets=torch.arange(pages + 1) * page, page_lengths=lengths,
+            page_classes=classes)
+        cache = R.build_three_precision_cache(key[rows].contiguous(), value[rows].contiguous(), plan, page_size=page)
+        return make_executor(cache, q.shape[1]).decode_f32(q.contiguous())
+
+    want = torch.cat([decode(slice(h, h + 1), query[:, 7 * h:7 * h + 7]) for h in range(heads)], dim=1)   # one head: aligned
+    if cap:
+        monkeypatch.setenv("R2K_GRID_CAP", str(cap))   # one CTA per head streams all of its tiles
+    assert_close(decode(slice(None), query), want.cpu(), "all heads against one at a time")
