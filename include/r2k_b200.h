@@ -323,6 +323,8 @@ int r2k_gather_rows(const void* src, int32_t num_kv_heads, int64_t src_rows, con
  * consecutive) or as one value per source row (`global_rows`, `logical_rows`).
  * Replaces build_three_precision_cache's packing (r2omni/sspa/runtime/precision_pool.py:611-746, 787-984).
  */
+enum { R2K_BUILD_OTHER_VALUES = 16 };   /* added to `dtype`: the values are of the other element type; bf16 pages hold them
+                                           rounded to the keys' type, which is the cache's */
 typedef struct R2KPage { int32_t dst, src; } R2KPage;
 typedef struct R2KBuild {
   const void* key; const void* value;

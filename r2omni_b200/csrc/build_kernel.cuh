@@ -91,7 +91,8 @@ __device__ __forceinline__ void build_keys(const R2KBuild& b, int chunk, int hea
   }
 }
 
-template <bool BF16>
+// BF16: the values' type; CACHE_BF16: the cache's.
+template <bool BF16, bool CACHE_BF16>
 __device__ __forceinline__ void build_values(const R2KBuild& b, int chunk, int head, const int* src_row) {
   const int warp = (threadIdx.x >> 5) - 4, lane = threadIdx.x & 31;
   const uint16_t* src = reinterpret_cast<const uint16_t*>(b.value) + (int64_t)head * b.rows * 128 + 4 * lane;
@@ -112,6 +113,11 @@ __device__ __forceinline__ void build_values(const R2KBuild& b, int chunk, int h
       for (int j = 0; j < 7; ++j) w[j] = w[j + 1];   // the next row moves to the front: one copy of the code for eight rows
       int row = chunk * kBuildRows + 32 * warp + i0 + k;
       if (row < b.n_fp) {
+        if (BF16 != CACHE_BF16) {
+          float x[4];
+          unpack4<BF16>(v, x);
+          v = CACHE_BF16 ? make_uint2(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3])) : make_uint2(pack_f16x2(x[0], x[1]), pack_f16x2(x[2], x[3]));
+        }
         *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(b.fp_v) + ((int64_t)head * b.n_fp + row) * 128 + 4 * lane) = v;
         continue;
       }
@@ -137,7 +143,7 @@ __device__ __forceinline__ void build_values(const R2KBuild& b, int chunk, int h
   }
 }
 
-template <bool BF16>
+template <bool BF16, bool VALUES_BF16>
 __global__ void __launch_bounds__(kBuildThreads, 2) build_cache_kernel(const __grid_constant__ BuildArgs a) {
   __shared__ int src_row[kBuildRows];
   __shared__ float range[4][128][2];
@@ -157,7 +163,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) build_cache_kernel(const __g
     }
     __syncthreads();
     if (threadIdx.x < 128) build_keys<BF16>(b, chunk, head, src_row, range);
-    else build_values<BF16>(b, chunk, head, src_row);
+    else build_values<VALUES_BF16, BF16>(b, chunk, head, src_row);
     return;
   }
   cta -= a.chunk_ctas;

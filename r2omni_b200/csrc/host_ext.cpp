@@ -129,7 +129,9 @@ py::tuple build_cache(const at::Tensor& key, const at::Tensor& value, const at::
                       int64_t page_size, int64_t k_block, int64_t v2_group, int64_t recent_capacity, int64_t append_capacity) {
   const c10::cuda::CUDAGuard guard(key.device());
   const int64_t h = key.size(0), rows = key.size(1), d = 128;
-  const int dtype = dtype_code(key.scalar_type());
+  if (value.device() != key.device()) throw py::value_error("key/value must share a device");
+  const int key_type = dtype_code(key.scalar_type()), value_type = dtype_code(value.scalar_type());
+  const int dtype = key_type == value_type ? key_type : key_type | R2K_BUILD_OTHER_VALUES;
   const at::Tensor cls_t = host_i64(page_classes), off_t = host_i64(page_offsets), len_t = host_i64(page_lengths);
   const int64_t n = cls_t.numel();
   if (off_t.numel() != n || len_t.numel() != n) throw py::value_error("page table columns differ in length");

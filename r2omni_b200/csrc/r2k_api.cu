@@ -762,7 +762,9 @@ int r2k_gather_rows(const void* src, int32_t num_kv_heads, int64_t src_rows, con
 
 int r2k_build_cache(const R2KBuild* build, void* stream) {
   if (build == nullptr) return R2K_ERR_NULL;
-  const R2KBuild& b = *build;
+  R2KBuild b = *build;
+  const bool other_values = (b.dtype & R2K_BUILD_OTHER_VALUES) != 0;
+  b.dtype &= ~R2K_BUILD_OTHER_VALUES;
   if ((b.rows > 0 && (!b.key || !b.value)) || !b.pages || !b.k_packed || !b.k_scale || !b.k_zero || !b.i2_packed || !b.i2_scale || !b.i2_zero ||
       !b.recent_k || !b.recent_v || !b.recent_len || !b.recent_global || !b.recent_logical || !b.recent_page_lengths)
     return R2K_ERR_NULL;
@@ -811,8 +813,10 @@ int r2k_build_cache(const R2KBuild* build, void* stream) {
   static_assert(kMaxFills == 13, "one per call above");
   if (ctas > 0x7fffffff) return R2K_ERR_GEOMETRY;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (b.dtype == R2K_DTYPE_BF16) build_cache_kernel<true><<<(unsigned)ctas, kBuildThreads, 0, st>>>(a);
-  else build_cache_kernel<false><<<(unsigned)ctas, kBuildThreads, 0, st>>>(a);
+  const bool bf16 = b.dtype == R2K_DTYPE_BF16;
+  const auto kernel = bf16 ? (other_values ? build_cache_kernel<true, false> : build_cache_kernel<true, true>)
+                           : (other_values ? build_cache_kernel<false, true> : build_cache_kernel<false, false>);
+  kernel<<<(unsigned)ctas, kBuildThreads, 0, st>>>(a);
   ++g_launches;
   return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
 }

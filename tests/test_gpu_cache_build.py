@@ -135,3 +135,38 @@ def test_rotation_of_unaligned_rows_and_ragged_sections(sections, shift, batch, 
     for a, b in zip(got, want):
         assert torch.equal(a.cpu().view(torch.int16), b.view(torch.int16))
     assert torch.equal(R.triton_fwht_128(k).cpu().view(torch.int16), R.triton_fwht_128(k.clone()).cpu().view(torch.int16))
+
+
+@pytest.mark.parametrize("key_dtype,value_dtype", [(torch.bfloat16, torch.float16), (torch.float16, torch.bfloat16)])
+def test_values_of_the_other_element_type(key_dtype, value_dtype):
+    """Keys and values of different 16-bit types: each is read as what it is; bf16 pages hold the values rounded to the
+    cache's (the keys') type."""
+    lengths, classes = [16, 3, 16, 16, 1, 16, 7, 16], [5, 2, 1, 1, 2, 0, 5, 2]
+    total, plan = sum(lengths), _plan(classes, lengths)
+    g = torch.Generator().manual_seed(total)
+    key = torch.randn(2, total, 128, generator=g).to(key_dtype).cuda()
+    value = torch.randn(2, total, 128, generator=g).to(value_dtype).cuda()
+    a = R.build_three_precision_cache(key, value, plan, page_size=16).arenas
+    same = R.build_three_precision_cache(value, value, plan, page_size=16).arenas
+    keys = R.build_three_precision_cache(key, key, plan, page_size=16).arenas
+    for name in ("k_packed", "k_scale", "k_zero"):
+        assert torch.equal(getattr(a, name), getattr(keys, name)), name
+    for name in ("i4_packed", "i4_scale", "i2_packed", "i2_scale", "i2_zero"):
+        assert torch.equal(getattr(a, name), getattr(same, name)), name
+    fp = tier_sorted_tokens(plan)[0]
+    assert a.fp_v.dtype == key_dtype and torch.equal(a.fp_v[0].cpu(), value.cpu()[:, fp].to(key_dtype))
+
+
+def test_values_of_no_cache_type_are_refused():
+    plan = _plan([2, 1], [16, 16])
+    key = torch.zeros(1, 32, 128, dtype=torch.bfloat16, device="cuda")
+    for value in (key.float(), key.double()):
+        with pytest.raises(ValueError):
+            R.build_three_precision_cache(key, value, plan, page_size=16)
+
+
+def test_values_on_another_device_are_refused():
+    plan = _plan([2, 1], [16, 16])
+    key = torch.zeros(1, 32, 128, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(ValueError):
+        R.build_three_precision_cache(key, key.cpu(), plan, page_size=16)
