@@ -34,11 +34,11 @@ int dtype_code(at::ScalarType t) {
 // ---------------------------------------------------------------------------
 // decode step
 // ---------------------------------------------------------------------------
-// Everything about an executor's launch that does not change from step to step.  The geometry and view structs are the ones
-// the Python side holds (and keeps alive); the output tensor is the workspace's.
+// Everything about an executor's launch that does not change from step to step: copies of its geometry and of the cache's
+// addresses (the Python side makes a new Step when these are taken again), and the workspace, kept alive.
 struct Step {
-  R2KGeom* geom;
-  const R2KCacheView* view;
+  R2KGeom geom;
+  R2KCacheView view;
   void* workspace;
   size_t workspace_bytes;
   at::Tensor buffer, output;
@@ -48,9 +48,9 @@ struct Step {
   int64_t batch, heads, kv_numel;
 
   Step(uintptr_t geom_, uintptr_t view_, const at::Tensor& buffer_, const at::Tensor& output_, const at::Tensor& like, uint32_t flags_)
-      : geom(reinterpret_cast<R2KGeom*>(geom_)), view(reinterpret_cast<const R2KCacheView*>(view_)), workspace(buffer_.data_ptr()),
+      : geom(*reinterpret_cast<const R2KGeom*>(geom_)), view(*reinterpret_cast<const R2KCacheView*>(view_)), workspace(buffer_.data_ptr()),
         workspace_bytes((size_t)buffer_.numel()), buffer(buffer_), output(output_), dtype(like.scalar_type()), device(like.device()), flags(flags_),
-        batch(geom->batch), heads(geom->num_q_heads), kv_numel((int64_t)geom->batch * geom->num_kv_heads * 128) {}
+        batch(geom.batch), heads(geom.num_q_heads), kv_numel((int64_t)geom.batch * geom.num_kv_heads * 128) {}
 
   // ap filled from (k, v); the indices are the caller's business
   void rows(R2KAppend& ap, const at::Tensor& k, const at::Tensor& v) const {
@@ -61,20 +61,21 @@ struct Step {
     ap.v = v.data_ptr();
   }
 
-  void launch(const at::Tensor& query, const R2KAppend* ap, int32_t n_i2) {
+  void launch(const at::Tensor& query, const R2KAppend* ap, int32_t n_i2) const {
     const bool four = query.dim() == 4 && query.size(2) == 1;   // [B,Hq,1,128]
     if (query.dim() == 4 && query.size(2) > 1) return launch(query.select(2, 0), ap, n_i2);   // its first token's rows
     if (!((query.dim() == 3 && query.size(2) == 128) || (four && query.size(3) == 128)) || query.size(0) != batch ||
         query.size(1) != heads || query.device() != device || query.scalar_type() != dtype || !query.is_contiguous())
       throw py::value_error("query does not match prepared split-K executor");
-    geom->n_i2 = n_i2;   // the only extent that moves during generation (flushes)
-    const int status = r2k_decode(geom, view, query.data_ptr(), ap, workspace, workspace_bytes, output.data_ptr(), flags,
+    R2KGeom now = geom;
+    now.n_i2 = n_i2;   // the only extent that moves during generation (flushes)
+    const int status = r2k_decode(&now, &view, query.data_ptr(), ap, workspace, workspace_bytes, output.data_ptr(), flags,
                                   at::cuda::getCurrentCUDAStream(device.index()).stream());
     if (status != R2K_OK) check(status, "r2k_decode");
   }
-  void plain(const at::Tensor& query, int32_t n_i2) { launch(query, nullptr, n_i2); }
+  void plain(const at::Tensor& query, int32_t n_i2) const { launch(query, nullptr, n_i2); }
   void append(const at::Tensor& query, const at::Tensor& k, const at::Tensor& v, int64_t global_index, int64_t logical_position,
-                    int32_t n_i2) {
+              int32_t n_i2) const {
     R2KAppend ap{};
     rows(ap, k, v);
     ap.global_index = global_index;

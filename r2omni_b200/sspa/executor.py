@@ -125,7 +125,7 @@ class SplitKExecutor:
         self._host_staging, self._host_pair = None, None
         # fp16 caches: the kernel's element type is fp16, the operator's output is bf16
         self._flags = (L.FLAG_OUTPUT_HADAMARD if self.output_hadamard else 0) | (0 if arenas.dtype == torch.bfloat16 else L.FLAG_OUT_BF16)
-        self._step, self._batched = None, arenas.batch > 1
+        self._step, self._step_view, self._batched = None, None, arenas.batch > 1
         self._ring_capacity, self._static_tokens = arenas.recent_capacity, arenas.n_fp + arenas.n_i4
 
     @property
@@ -192,9 +192,9 @@ class SplitKExecutor:
         return self._append_ref
 
     def _make_step(self):
-        """The native per-step call: checks, argument block and launch (csrc/host_ext.cpp)."""
-        view = self.arenas.view()
-        self._view_obj, self._view_ref = view, C.byref(view)
+        """The native per-step call: checks, argument block and launch (csrc/host_ext.cpp).  It copies the addresses of
+        the view that `_step_view` records; the other ways to launch keep a record of their own (`_view_obj`)."""
+        view = self._step_view = self.arenas.view()
         self._step = host().Step(C.addressof(self._geom), C.addressof(view), self.workspace.buffer, self.workspace.output,
                                  self.arenas.recent_k, self._flags)
         return self._step
@@ -202,7 +202,7 @@ class SplitKExecutor:
     def __call__(self, query: torch.Tensor, append=None) -> torch.Tensor:
         a = self.arenas
         step = self._step
-        if step is None or a._view is not self._view_obj:
+        if step is None or a._view is not self._step_view:
             step = self._make_step()
         output = self.workspace.output
         if append is None:

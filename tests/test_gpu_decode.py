@@ -381,3 +381,17 @@ def test_host_buffer_step_matches_device_call_and_oracle():
         ex_host.step_host(host_in[: hq * 128], host_out, append_indices=(0, 0))   # rows missing
     with pytest.raises(ValueError):
         ex_host.step_host(host_in.cuda(), host_out)
+
+
+def test_rebound_tensor_after_a_launch_of_another_kind():
+    """A cache tensor replaced between calls: whoever launches first after the addresses are taken again, all follow."""
+    _, gcache, _, _, queries = both_caches(8, hq=16, hkv=2, tokens=512, page=64, classes=seeded_classes(8, 8), appends=1)
+    a, q = gcache.arenas, queries[0].cuda()
+    ex = make_executor(gcache, 16)
+    ex(q)
+    old = a.k_packed
+    a.k_packed = old.flip(2).contiguous()
+    old.fill_(0x77)
+    a._view = None
+    want = ex.decode_f32(q)
+    assert torch.equal(ex(q), want.to(torch.bfloat16))
