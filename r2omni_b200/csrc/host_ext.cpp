@@ -35,21 +35,21 @@ int dtype_code(at::ScalarType t) {
 // decode step
 // ---------------------------------------------------------------------------
 // Everything about an executor's launch that does not change from step to step: copies of its geometry and of the cache's
-// addresses (the Python side makes a new Step when these are taken again), and the workspace, kept alive.
+// addresses (the Python side makes a new Step when these are taken again), and the workspace, kept alive.  The output tensor
+// and the flags are the caller's to change and come with every call.
 struct Step {
   R2KGeom geom;
   R2KCacheView view;
   void* workspace;
   size_t workspace_bytes;
-  at::Tensor buffer, output;
+  at::Tensor buffer;
   at::ScalarType dtype;
   c10::Device device;
-  uint32_t flags;
   int64_t batch, heads, kv_numel;
 
-  Step(uintptr_t geom_, uintptr_t view_, const at::Tensor& buffer_, const at::Tensor& output_, const at::Tensor& like, uint32_t flags_)
+  Step(uintptr_t geom_, uintptr_t view_, const at::Tensor& buffer_, const at::Tensor& like)
       : geom(*reinterpret_cast<const R2KGeom*>(geom_)), view(*reinterpret_cast<const R2KCacheView*>(view_)), workspace(buffer_.data_ptr()),
-        workspace_bytes((size_t)buffer_.numel()), buffer(buffer_), output(output_), dtype(like.scalar_type()), device(like.device()), flags(flags_),
+        workspace_bytes((size_t)buffer_.numel()), buffer(buffer_), dtype(like.scalar_type()), device(like.device()),
         batch(geom.batch), heads(geom.num_q_heads), kv_numel((int64_t)geom.batch * geom.num_kv_heads * 128) {}
 
   // ap filled from (k, v); the indices are the caller's business
@@ -61,26 +61,30 @@ struct Step {
     ap.v = v.data_ptr();
   }
 
-  void launch(const at::Tensor& query, const R2KAppend* ap, int32_t n_i2) const {
+  void launch(const at::Tensor& query, const R2KAppend* ap, const at::Tensor& output, uint32_t flags, int32_t n_i2) const {
     const bool four = query.dim() == 4 && query.size(2) == 1;   // [B,Hq,1,128]
-    if (query.dim() == 4 && query.size(2) > 1) return launch(query.select(2, 0), ap, n_i2);   // its first token's rows
+    if (query.dim() == 4 && query.size(2) > 1) return launch(query.select(2, 0), ap, output, flags, n_i2);   // its first token's rows
     if (!((query.dim() == 3 && query.size(2) == 128) || (four && query.size(3) == 128)) || query.size(0) != batch ||
         query.size(1) != heads || query.device() != device || query.scalar_type() != dtype || !query.is_contiguous())
       throw py::value_error("query does not match prepared split-K executor");
+    if (output.numel() != batch * heads * 128 || output.scalar_type() != at::kBFloat16 || output.device() != device || !output.is_contiguous())
+      throw py::value_error("workspace output does not match prepared split-K executor");
     R2KGeom now = geom;
     now.n_i2 = n_i2;   // the only extent that moves during generation (flushes)
     const int status = r2k_decode(&now, &view, query.data_ptr(), ap, workspace, workspace_bytes, output.data_ptr(), flags,
                                   at::cuda::getCurrentCUDAStream(device.index()).stream());
     if (status != R2K_OK) check(status, "r2k_decode");
   }
-  void plain(const at::Tensor& query, int32_t n_i2) const { launch(query, nullptr, n_i2); }
+  void plain(const at::Tensor& query, const at::Tensor& output, uint32_t flags, int32_t n_i2) const {
+    launch(query, nullptr, output, flags, n_i2);
+  }
   void append(const at::Tensor& query, const at::Tensor& k, const at::Tensor& v, int64_t global_index, int64_t logical_position,
-              int32_t n_i2) const {
+              const at::Tensor& output, uint32_t flags, int32_t n_i2) const {
     R2KAppend ap{};
     rows(ap, k, v);
     ap.global_index = global_index;
     ap.logical_position = logical_position;
-    launch(query, &ap, n_i2);
+    launch(query, &ap, output, flags, n_i2);
   }
 };
 
@@ -394,7 +398,7 @@ std::vector<at::Tensor> qkv_prologue(const at::Tensor& query, const at::Tensor& 
 
 PYBIND11_MODULE(_r2k_host, m) {
   py::class_<Step>(m, "Step")
-      .def(py::init<uintptr_t, uintptr_t, const at::Tensor&, const at::Tensor&, const at::Tensor&, uint32_t>())
+      .def(py::init<uintptr_t, uintptr_t, const at::Tensor&, const at::Tensor&>())
       .def("plain", &Step::plain)
       .def("append", &Step::append);
   m.def("build_cache", &build_cache);

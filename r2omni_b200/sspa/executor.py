@@ -120,11 +120,12 @@ class SplitKExecutor:
         self._geom_ref = C.byref(self._geom)
         self._append_ref = C.byref(self._append)
         self._view_obj, self._view_ref = None, None
+        self._ws_buffer = workspace.buffer   # scratch of every launch, whatever becomes of `workspace`
         self._ws_ptr, self._ws_size = workspace.buffer.data_ptr(), workspace.buffer.numel()
         self._qshape = (arenas.batch, self.num_query_heads, 128)
         self._host_staging, self._host_pair = None, None
         # fp16 caches: the kernel's element type is fp16, the operator's output is bf16
-        self._flags = (L.FLAG_OUTPUT_HADAMARD if self.output_hadamard else 0) | (0 if arenas.dtype == torch.bfloat16 else L.FLAG_OUT_BF16)
+        self._out_bf16 = 0 if arenas.dtype == torch.bfloat16 else L.FLAG_OUT_BF16
         self._step, self._step_view, self._batched = None, None, arenas.batch > 1
         self._ring_capacity, self._static_tokens = arenas.recent_capacity, arenas.n_fp + arenas.n_i4
 
@@ -195,8 +196,7 @@ class SplitKExecutor:
         """The native per-step call: checks, argument block and launch (csrc/host_ext.cpp).  It copies the addresses of
         the view that `_step_view` records; the other ways to launch keep a record of their own (`_view_obj`)."""
         view = self._step_view = self.arenas.view()
-        self._step = host().Step(C.addressof(self._geom), C.addressof(view), self.workspace.buffer, self.workspace.output,
-                                 self.arenas.recent_k, self._flags)
+        self._step = host().Step(C.addressof(self._geom), C.addressof(view), self._ws_buffer, self.arenas.recent_k)
         return self._step
 
     def __call__(self, query: torch.Tensor, append=None) -> torch.Tensor:
@@ -205,19 +205,20 @@ class SplitKExecutor:
         if step is None or a._view is not self._step_view:
             step = self._make_step()
         output = self.workspace.output
+        flags = self._out_bf16 | L.FLAG_OUTPUT_HADAMARD if self.output_hadamard else self._out_bf16
         if append is None:
             if a.recent_len == 0 and self._static_tokens + a.i2_active == 0:
                 raise ValueError("four-quadrant cache has no surviving tokens")
-            step.plain(query, a.i2_active)
+            step.plain(query, output, flags, a.i2_active)
             return output
         k, v, global_index, logical_position = append
         if a.recent_len >= self._ring_capacity:
             raise RuntimeError("prepared executor cannot fuse an append into a full Recent-FP pool")
         if type(global_index) is int and type(logical_position) is int:
-            step.append(query, k, v, global_index, logical_position, a.i2_active)
+            step.append(query, k, v, global_index, logical_position, output, flags, a.i2_active)
         else:   # per-request or device-resident indices
             query = self._check_query(query)
-            self._launch(query, self._make_append(append, query), output.data_ptr(), self._flags)
+            self._launch(query, self._make_append(append, query), output.data_ptr(), flags)
         if self._batched:
             a.recent_len += 1
         return output

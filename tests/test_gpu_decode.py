@@ -395,3 +395,24 @@ def test_rebound_tensor_after_a_launch_of_another_kind():
     a._view = None
     want = ex.decode_f32(q)
     assert torch.equal(ex(q), want.to(torch.bfloat16))
+
+
+def test_attributes_changed_after_preparation_count():
+    """`output_hadamard`, the workspace and its output tensor are the caller's to change: every way to launch reads them."""
+    _, gcache, new_k, new_v, queries = both_caches(8, hq=16, hkv=2, tokens=512, page=64, classes=seeded_classes(8, 8), appends=2)
+    q = queries[0].cuda()
+    plain, rotated = make_executor(gcache, 16), make_executor(gcache, 16, output_hadamard=True)
+    want, want_rotated = plain(q).clone(), rotated(q).clone()
+    plain.output_hadamard = True
+    assert torch.equal(plain(q), want_rotated)
+    plain.output_hadamard = False
+    mine = torch.zeros_like(plain.workspace.output)
+    plain.workspace.output = mine
+    assert plain(q) is mine and torch.equal(mine, want)
+    plain.workspace = R.allocate_splitk_workspace(gcache, num_query_heads=16)
+    mine.zero_()
+    got = plain(q)
+    assert got is plain.workspace.output and torch.equal(got, want) and not mine.any()
+    plain.output_hadamard = True
+    k, v = new_k[0].unsqueeze(0).contiguous().cuda(), new_v[0].unsqueeze(0).contiguous().cuda()
+    assert torch.equal(plain(q, append=(k, v, 512, 512)).clone(), make_executor(gcache, 16, output_hadamard=True)(q))
