@@ -129,9 +129,10 @@ inline int tier_of(int64_t cls) { return cls == 1 || cls == 3 || cls == 4 ? 0 : 
 
 // build_three_precision_cache behind its argument checks.  Returns (tensors in the order of `names` on the Python side,
 // n_fp, n_i4, n_i2).
-py::tuple build_cache(const at::Tensor& key, const at::Tensor& value, const at::Tensor& page_classes, const at::Tensor& page_offsets,
-                      const at::Tensor& page_lengths, const at::Tensor& global_index, const at::Tensor& logical_position,
-                      int64_t page_size, int64_t k_block, int64_t v2_group, int64_t recent_capacity, int64_t append_capacity) {
+std::tuple<std::vector<at::Tensor>, int64_t, int64_t, int64_t> build_cache(
+    const at::Tensor& key, const at::Tensor& value, const at::Tensor& page_classes, const at::Tensor& page_offsets,
+    const at::Tensor& page_lengths, const at::Tensor& global_index, const at::Tensor& logical_position,
+    int64_t page_size, int64_t k_block, int64_t v2_group, int64_t recent_capacity, int64_t append_capacity) {
   const c10::cuda::CUDAGuard guard(key.device());
   const int64_t h = key.size(0), rows = key.size(1), d = 128;
   if (value.device() != key.device()) throw py::value_error("key/value must share a device");
@@ -242,7 +243,7 @@ py::tuple build_cache(const at::Tensor& key, const at::Tensor& value, const at::
   b.fp_global = (int64_t*)ptr(17); b.fp_logical = (int64_t*)ptr(18); b.i4_global = (int64_t*)ptr(19); b.i4_logical = (int64_t*)ptr(20);
   b.evicted_global = (int64_t*)ptr(21);
   check(r2k_build_cache(&b, at::cuda::getCurrentCUDAStream().stream()), "r2k_build_cache");   // without tokens, too: it clears the cache
-  return py::make_tuple(std::move(t), n_fp, n_i4, n_i2);
+  return {std::move(t), n_fp, n_i4, n_i2};
 }
 
 // ---------------------------------------------------------------------------
@@ -396,13 +397,17 @@ std::vector<at::Tensor> qkv_prologue(const at::Tensor& query, const at::Tensor& 
 
 }  // namespace
 
+// The interpreter is left to other threads for the length of a call (no function here touches a Python object): a launch
+// waits while the device's queue is full, an allocation may wait for the driver.
+using unlocked = py::call_guard<py::gil_scoped_release>;
+
 PYBIND11_MODULE(_r2k_host, m) {
   py::class_<Step>(m, "Step")
       .def(py::init<uintptr_t, uintptr_t, const at::Tensor&, const at::Tensor&>())
-      .def("plain", &Step::plain)
-      .def("append", &Step::append);
-  m.def("build_cache", &build_cache);
-  m.def("fwht", &fwht);
-  m.def("qk_mrope", &qk_mrope);
-  m.def("qkv_prologue", &qkv_prologue);
+      .def("plain", &Step::plain, unlocked())
+      .def("append", &Step::append, unlocked());
+  m.def("build_cache", &build_cache, unlocked());
+  m.def("fwht", &fwht, unlocked());
+  m.def("qk_mrope", &qk_mrope, unlocked());
+  m.def("qkv_prologue", &qkv_prologue, unlocked());
 }
