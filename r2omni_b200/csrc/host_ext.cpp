@@ -144,7 +144,8 @@ std::tuple<std::vector<at::Tensor>, int64_t, int64_t, int64_t> build_cache(
   const int64_t *cls = cls_t.data_ptr<int64_t>(), *off = off_t.data_ptr<int64_t>(), *len = len_t.data_ptr<int64_t>();
   int64_t tokens[4] = {0, 0, 0, 0}, total = 0;
   for (int64_t i = 0; i < n; ++i) {
-    if (len[i] < 0 || off[i] < 0 || off[i] + len[i] > rows) throw py::value_error("page lies outside the keys and values");
+    if (len[i] == 0) continue;   // its place is of no consequence
+    if (len[i] < 0 || off[i] < 0 || len[i] > rows || off[i] > rows - len[i]) throw py::value_error("page lies outside the keys and values");
     tokens[tier_of(cls[i])] += len[i];
     total += len[i];
   }
@@ -160,6 +161,7 @@ std::tuple<std::vector<at::Tensor>, int64_t, int64_t, int64_t> build_cache(
     logical = host_i64(logical);
     const int64_t *g = global.data_ptr<int64_t>(), *l = logical.data_ptr<int64_t>();
     for (int64_t i = 0; i < n && by_page; ++i) {
+      if (len[i] < 2) continue;
       const int64_t *gp = g + off[i], *lp = l + off[i];
       int64_t odd = 0;
       for (int64_t k = 1; k < len[i]; ++k) odd |= (gp[k] - gp[0] - k) | (lp[k] - lp[0] - k);

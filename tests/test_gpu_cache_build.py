@@ -209,3 +209,12 @@ def test_build_time_does_not_grow_with_the_square_of_the_pages():
         torch.cuda.synchronize()
         times.append(begin.elapsed_time(end))
     assert min(times) < 20.0, times
+
+
+def test_pages_without_tokens_may_start_anywhere():
+    plan = _plan([2, 1, 5], [16, 0, 16])
+    object.__setattr__(plan, "page_offsets", torch.tensor([0, 4711, 16]))
+    key = torch.randn(1, 32, 128, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    a = R.build_three_precision_cache(key, key, plan, page_size=16).arenas
+    b = R.build_three_precision_cache(key, key, _plan([2, 1, 5], [16, 0, 16]), page_size=16).arenas
+    assert torch.equal(a.k_packed, b.k_packed) and torch.equal(a.i2_packed, b.i2_packed) and torch.equal(a.i4_packed, b.i4_packed)
