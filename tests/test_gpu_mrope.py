@@ -113,3 +113,17 @@ def test_one_launch_prologue_rejects_bad_arguments():
         R.qwen_qkv_prologue(q, k, v, cos, sin, (16, 24, 20))
     with pytest.raises(RuntimeError):
         R.qwen_qkv_prologue(q.cpu(), k.cpu(), v.cpu(), cos.cpu(), sin.cpu(), (16, 24, 24))
+
+
+def test_outputs_given_as_any_iterable():
+    q, k, cos, sin = _inputs(2, 4, 2, 1, torch.bfloat16, torch.float32, seed=3)
+    qd, kd, cd, sd = q.cuda(), k.cuda(), cos.cuda(), sin.cuda()
+    want = R.qwen_qk_mrope(qd, kd, cd, sd, (16, 24, 24))
+    outs = [torch.empty_like(qd), torch.empty_like(kd)]
+    for given in (outs, tuple(outs), iter(outs)):
+        got = R.qwen_qk_mrope(qd, kd, cd, sd, (16, 24, 24), output=given)
+        assert got[0] is outs[0] and got[1] is outs[1] and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    rows = [t.flatten(1).unsqueeze(1) for t in (qd, kd, kd)]
+    outs = [torch.empty_like(t) for t in (qd, kd, kd)]
+    got = R.qwen_qkv_prologue(*rows, cd, sd, (16, 24, 24), output=iter(outs))
+    assert all(a is b for a, b in zip(got, outs)) and torch.equal(outs[0], want[0]) and torch.equal(outs[2], kd)
