@@ -416,3 +416,25 @@ def test_attributes_changed_after_preparation_count():
     plain.output_hadamard = True
     k, v = new_k[0].unsqueeze(0).contiguous().cuda(), new_v[0].unsqueeze(0).contiguous().cuda()
     assert torch.equal(plain(q, append=(k, v, 512, 512)).clone(), make_executor(gcache, 16, output_hadamard=True)(q))
+
+
+@pytest.mark.parametrize("hkv,grid_cap", [(20, None), (2, None), (2, 5), (2, 3)])
+def test_residual_tiles_alone_on_their_ctas(hkv, grid_cap, monkeypatch):
+    """One packed tile and two residual tiles per head, spread so that the second residual tile is all a CTA has (20 heads:
+    one tile per CTA; 2 heads: clusters, or five or three CTAs in all), at every fill of the window: a tile without rows is
+    still handed over, the appended rows land where they belong and the length moves by one per step."""
+    if grid_cap:
+        monkeypatch.setenv("R2K_GRID_CAP", str(grid_cap))
+    hq = 2 * hkv
+    ocache, gcache, new_k, new_v, queries = both_caches(77, hq=hq, hkv=hkv, tokens=64, page=32, classes=torch.tensor([2, 2]),
+                                                        appends=128, append_capacity=128)
+    ex = make_executor(gcache, hq)
+    q, k, v = queries[0].cuda(), new_k.cuda(), new_v.cuda()
+    for i in range(128):
+        out = ex.decode_f32(q, append=(k[i].unsqueeze(0).contiguous(), v[i].unsqueeze(0).contiguous(), 64 + i, 64 + i))
+        gcache.recent_fp_pool.active_length += 1
+        O.append_token(ocache, new_k[i], new_v[i], 64 + i, 64 + i)
+        if i in (0, 1, 30, 62, 63, 64, 65, 126, 127):
+            assert_close(out, O.decode_fp32(queries[0].float(), ocache), f"append {i}")
+    arena_equal(ocache, gcache)
+    assert int(gcache.arenas.recent_len_device[0]) == 128 and ex.device_status() == 0
