@@ -132,6 +132,12 @@ int r2k_decode_workspace_bytes(const R2KGeom* geom, size_t* bytes);
  * another on a stream, as long as it is large enough for each of them.          */
 int r2k_decode_workspace_init(void* workspace, size_t bytes, void* stream);
 
+/* How r2k_decode (world = 1) or r2k_decode_exchange would lay a launch of this geometry and these flags out: the number of
+ * CTAs and the CTAs of a cluster (0: no clusters).  For the current device, or, with sms > 0 (no device needed), for
+ * one with that many SMs on which `clusters` clusters fit at once.  A launch that writes the state rows and the fused
+ * exchange have the same CTAs, and with them the same bits.                                                          */
+int r2k_decode_plan(const R2KGeom* geom, uint32_t flags, int32_t world, int32_t sms, int32_t clusters, int32_t* ctas, int32_t* cluster);
+
 /*
  * One decode step over a batch of packed caches: split-K partial attention over
  * the INT4 keys and bf16/INT4/INT2 value pools plus the residual window, exact

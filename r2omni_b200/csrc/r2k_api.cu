@@ -99,11 +99,10 @@ int windows(int a0, int n, int tile, int* first) {
   return (a0 + n + tile - 1) / tile - a0 / tile;
 }
 
-// Everything the kernel derives from the geometry; shared by workspace sizing and the launch.
-int derive(const R2KGeom* g, DecodeParams* p) {
-  DeviceInfo* dev;
-  int rc = device_info(&dev);
-  if (rc) return rc;
+// Everything the kernel derives from the geometry for a device of `sms` SMs that holds `clusters` decode clusters; shared by
+// workspace sizing and the launch.  `rows`: the launch ends in un-normalised rows for a merge across ranks.  The fused
+// exchange and the launch that writes the rows out share one layout, so that both give the same bits.
+int derive(const R2KGeom* g, bool rows, int sms, int clusters, DecodeParams* p) {
   std::memset(p, 0, sizeof(*p));
   p->g = *g;
   p->gqa = g->num_q_heads / g->num_kv_heads;
@@ -143,7 +142,7 @@ int derive(const R2KGeom* g, DecodeParams* p) {
   }
   p->cF = w[0]; p->c4 = w[1]; p->c2 = w[2]; p->cR = w[3];
   const int64_t total_units = (int64_t)p->units * p->bh_total;
-  int64_t cap = (int64_t)dev->sms * kCtasPerSm;
+  int64_t cap = (int64_t)sms * kCtasPerSm;
   const int env_cap = grid_cap_from_env();
   if (env_cap > 0 && env_cap < cap) cap = env_cap;
   p->grid = (int)(total_units < cap ? total_units : cap);
@@ -164,8 +163,9 @@ int derive(const R2KGeom* g, DecodeParams* p) {
   // request x 2 heads take 90.2 us without and 76.0 with clusters at 5000 tokens (4.3 us of tile weight more per CTA),
   // 89.2 and 94.9 at 6500 (6.1 us).  Room: at most two thirds of the clusters that fit, so that some of the next launch's
   // come in and fetch while this one finishes; 12 heads of 3000 tokens took 88.6 us without and 98.0 with clusters.
-  if (p->grid > p->bh_total && 3 * p->bh_total <= 2 * dev->clusters && kCluster * p->bh_total <= cap && p->c_bh >= (uint32_t)kCluster &&
-      head_ns / kCluster - head_ns / per_head < 5000.0) {
+  // The fused exchange merges through the workspace and saves nothing by it, so `rows` has the line of the rule below.
+  if (p->grid > p->bh_total && 3 * p->bh_total <= 2 * clusters && kCluster * p->bh_total <= cap && p->c_bh >= (uint32_t)kCluster &&
+      head_ns / kCluster - head_ns / per_head < (rows ? 3000.0 : 5000.0)) {
     p->grid = kCluster * p->bh_total;
     p->cluster = 1;
   }
@@ -185,6 +185,12 @@ int derive(const R2KGeom* g, DecodeParams* p) {
   const float sm = g->sm_scale > 0.f ? g->sm_scale : 0.08838834764831845f;
   p->qscale = sm * 1.4426950408889634f;
   return R2K_OK;
+}
+
+int derive(const R2KGeom* g, bool rows, DecodeParams* p) {
+  DeviceInfo* dev;
+  const int rc = device_info(&dev);
+  return rc ? rc : derive(g, rows, dev->sms, dev->clusters, p);
 }
 
 size_t counters_bytes(const DecodeParams& p) {
@@ -374,10 +380,28 @@ int r2k_decode_workspace_bytes(const R2KGeom* geom, size_t* bytes) {
   if (bytes == nullptr) return R2K_ERR_NULL;
   int rc = check_geom(geom);
   if (rc) return rc;
-  DecodeParams p;
-  rc = derive(geom, &p);
+  *bytes = 0;
+  for (int rows = 0; rows < 2; ++rows) {   // a workspace serves launches of either layout
+    DecodeParams p;
+    rc = derive(geom, rows != 0, &p);
+    if (rc) return rc;
+    const size_t need = workspace_need(p);
+    if (need > *bytes) *bytes = need;
+  }
+  return R2K_OK;
+}
+
+int r2k_decode_plan(const R2KGeom* geom, uint32_t flags, int32_t world, int32_t sms, int32_t clusters, int32_t* ctas, int32_t* cluster) {
+  if (ctas == nullptr || cluster == nullptr) return R2K_ERR_NULL;
+  int rc = check_geom(geom);
   if (rc) return rc;
-  *bytes = workspace_need(p);
+  if (sms < 0 || clusters < 0 || world < 1) return R2K_ERR_GEOMETRY;
+  const bool rows = (flags & R2K_FLAG_OUT_STATE) || world > 1;
+  DecodeParams p;
+  rc = sms > 0 ? derive(geom, rows, sms, clusters, &p) : derive(geom, rows, &p);
+  if (rc) return rc;
+  *ctas = p.grid;
+  *cluster = p.cluster && world == 1 ? kCluster : 0;
   return R2K_OK;
 }
 
@@ -400,7 +424,7 @@ static int decode_impl(const R2KGeom* geom, const R2KCacheView* view, const void
   int rc = check_geom(geom);
   if (rc) return rc;
   DecodeParams p;
-  rc = derive(geom, &p);
+  rc = derive(geom, (flags & R2K_FLAG_OUT_STATE) || (ex != nullptr && ex->world > 1), &p);
   if (rc) return rc;
   if (workspace_bytes < workspace_need(p)) return R2K_ERR_WORKSPACE;
   if (!aligned16(workspace) || !aligned16(q) || !aligned16(out)) return R2K_ERR_ALIGNMENT;

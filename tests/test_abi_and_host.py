@@ -164,3 +164,54 @@ def test_step_byte_model_counts_every_stream():
     sys.path.insert(0, ROOT)
     import bench
     assert bench.algorithmic_bytes(64, 128, 64, 0, 1, append=False) == want
+
+
+def _geom(tokens, hkv=2, batch=1, ring=128):
+    g = L.Geom()
+    g.batch, g.num_q_heads, g.num_kv_heads, g.head_dim = batch, 8 * hkv, hkv, 128
+    g.dtype, g.page_size, g.k_block, g.v2_group = L.DTYPE_BF16, 32, 32, 32
+    g.n_i4 = g.i4_capacity = tokens
+    g.k_off_i4, g.k_off_i2, g.k_capacity = 0, tokens, -(-tokens // 128) * 128
+    g.recent_capacity = ring
+    return g
+
+
+def _plan(lib, g, flags=0, world=1):
+    ctas, cluster = C.c_int32(), C.c_int32()
+    assert lib.r2k_decode_plan(C.byref(g), C.c_uint32(flags), world, 148, 18, C.byref(ctas), C.byref(cluster)) == 0
+    return ctas.value, cluster.value
+
+
+@pytest.mark.parametrize("hkv,batch", [(1, 1), (2, 1), (4, 1), (2, 3), (8, 1)])
+def test_launch_layout_of_small_caches(lib, hkv, batch):
+    """Where the shared-memory merge saves a merge through L2, eight CTAs per head may stream longer than the grid they
+    replace; where it does not (the fused exchange), only as much longer as nine CTAs per head may.  The launch that
+    writes the rows for a merge across ranks has the exchange's CTAs."""
+    heads = hkv * batch
+    seen = set()
+    for tokens in list(range(32, 16384, 224)) + [4096, 5000, 6500]:
+        g = _geom(tokens, hkv, batch)
+        (plain, cluster), state, exchange = _plan(lib, g), _plan(lib, g, L.FLAG_OUT_STATE), _plan(lib, g, world=2)
+        assert exchange == (state[0], 0) and cluster in (0, 8) and (cluster == 0 or plain == 8 * heads)
+        tiles = -(-tokens // 256)
+        full = min(148, (tiles + 2) * heads)   # two residual tiles; CTAs with a tile each, or every SM
+        full = full // heads * heads if full >= 2 * heads and full // heads * heads * 20 >= full * 19 else full
+        longer = (tiles * 2110.0 + 2 * 500.0) * (1 / 8 - heads / full)
+        if exchange[0] == 8 * heads and full > 8 * heads:
+            assert longer < 3000.0, (tokens, longer)
+        assert (state[1] == 8) == (full > heads and longer < 3000.0), (tokens, longer)
+        assert (cluster == 8) == (full > heads and longer < 5000.0), (tokens, longer)
+        seen.add((cluster, state[1]))
+    assert seen == {(8, 8), (8, 0), (0, 0)} or heads > 2
+
+
+def test_launch_layout_arguments(lib):
+    ctas, cluster = C.c_int32(), C.c_int32()
+    g = _geom(1024)
+    call = lambda *a: lib.r2k_decode_plan(*a)  # noqa: E731
+    assert call(None, C.c_uint32(0), 1, 148, 18, C.byref(ctas), C.byref(cluster)) == L.ERR_NULL
+    assert call(C.byref(g), C.c_uint32(0), 1, 148, 18, None, C.byref(cluster)) == L.ERR_NULL
+    assert call(C.byref(g), C.c_uint32(0), 0, 148, 18, C.byref(ctas), C.byref(cluster)) == L.ERR_GEOMETRY
+    assert call(C.byref(g), C.c_uint32(0), 1, -1, 18, C.byref(ctas), C.byref(cluster)) == L.ERR_GEOMETRY
+    g.head_dim = 64
+    assert call(C.byref(g), C.c_uint32(0), 1, 148, 18, C.byref(ctas), C.byref(cluster)) == L.ERR_GEOMETRY
