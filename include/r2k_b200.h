@@ -92,7 +92,9 @@ typedef struct R2KGeom {
  *   recent_global / recent_logical i64 [recent_capacity],
  *   recent_page_lengths i64 [recent_capacity / page_size]
  *             (r2omni/sspa/runtime/precision_pool.py:747-784)
- * Pointers of an empty pool may be NULL.
+ * Pointers of an empty pool may be NULL.  Payload and key arrays and their strides are multiples of 16 bytes; value
+ * scales and zero points may start at any multiple of their element.  A decode reads these in the 16-byte granules that
+ * they lie in, that is, up to 15 bytes on either side of a pool's rows (never across a page), and ignores what is not theirs.
  */
 typedef struct R2KCacheView {
   const uint8_t* k_packed;  const void* k_scale;  const uint8_t* k_zero;

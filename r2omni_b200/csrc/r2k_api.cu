@@ -445,6 +445,11 @@ static int decode_impl(const R2KGeom* geom, const R2KCacheView* view, const void
   if ((view->k_packed_bstride | view->k_scale_bstride | view->k_zero_bstride | view->fp_v_bstride | view->i4_packed_bstride |
        view->i2_packed_bstride) & 15)
     return R2K_ERR_ALIGNMENT;
+  // scales are read as what they are, at whatever multiple of their own size
+  const uintptr_t requests = geom->batch > 1 ? ~(uintptr_t)0 : 0;
+  if ((geom->n_i4 && ((reinterpret_cast<uintptr_t>(view->i4_scale) | ((uintptr_t)view->i4_scale_bstride & requests)) & 3)) ||
+      (geom->n_i2 && ((reinterpret_cast<uintptr_t>(view->i2_scale) | ((uintptr_t)view->i2_scale_bstride & requests)) & 1)))
+    return R2K_ERR_ALIGNMENT;
   p.v = *view;
   p.q = q;
   if (append != nullptr && append->k != nullptr) {

@@ -438,3 +438,14 @@ def test_residual_tiles_alone_on_their_ctas(hkv, grid_cap, monkeypatch):
             assert_close(out, O.decode_fp32(queries[0].float(), ocache), f"append {i}")
     arena_equal(ocache, gcache)
     assert int(gcache.arenas.recent_len_device[0]) == 128 and ex.device_status() == 0
+
+
+@pytest.mark.parametrize("name,off", [("i4_scale", 2), ("i4_scale", 1), ("i2_scale", 1)])
+def test_scales_off_their_own_alignment_are_refused(name, off):
+    _, gcache, _, _, queries = both_caches(5, hq=16, hkv=2, tokens=256, page=64, classes=torch.tensor([1, 2, 5, 2]), appends=1)
+    ex, q = make_executor(gcache, 16), queries[0].cuda()
+    out = torch.empty(1, 16, 128, device="cuda", dtype=torch.bfloat16)
+    geom, view = gcache.arenas.geom(16), L.CacheView.from_buffer_copy(gcache.arenas.view())
+    setattr(view, name, getattr(view, name) + off)
+    assert L.lib().r2k_decode(C.byref(geom), C.byref(view), q.data_ptr(), None, ex._ws_ptr, ex._ws_size, out.data_ptr(), 0,
+                              torch.cuda.current_stream().cuda_stream) == L.ERR_ALIGNMENT
