@@ -12,6 +12,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "lib", "libr2k_b200.so")
 HOST_LIB = os.path.join(PKG, "lib", "_r2k_host.so")
+HOST_TAG = os.path.join(PKG, "lib", "_r2k_host.tag")   # what the host module was built for
 HOST_SOURCE = "host_ext.cpp"
 SOURCES = ("r2k_api.cu",)
 HEADERS = ("decode.cuh", "decode_consumer.cuh", "decode_kernel.cuh", "device_utils.cuh", "pack_kernels.cuh", "build_kernel.cuh")
@@ -24,14 +25,28 @@ def _stale(target: str, sources) -> bool:
     return any(os.path.getmtime(d) > built for d in sources)
 
 
+def _host_tag() -> str:
+    import torch
+
+    return f"torch {torch.__version__}, {sys.implementation.cache_tag}"
+
+
+def host_stale() -> bool:
+    """Whether the host module is missing, older than its sources, or built for another torch or Python."""
+    if _stale(HOST_LIB, (os.path.join(CSRC, HOST_SOURCE), os.path.join(ROOT, "include", "r2k_b200.h"))) or not os.path.exists(HOST_TAG):
+        return True
+    with open(HOST_TAG) as f:
+        return f.read() != _host_tag()
+
+
 def _build_host(force: bool) -> None:
-    source, header = os.path.join(CSRC, HOST_SOURCE), os.path.join(ROOT, "include", "r2k_b200.h")
-    if not force and not _stale(HOST_LIB, (source, header)):
+    if not force and not host_stale():
         return
     import sysconfig
 
     import torch
 
+    source = os.path.join(CSRC, HOST_SOURCE)
     torch_dir = os.path.dirname(torch.__file__)
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     includes = (os.path.join(ROOT, "include"), os.path.join(torch_dir, "include"),
@@ -46,6 +61,8 @@ def _build_host(force: bool) -> None:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
         raise RuntimeError("g++ failed:\n" + proc.stdout + proc.stderr)
+    with open(HOST_TAG, "w") as f:
+        f.write(_host_tag())
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:

@@ -5,6 +5,7 @@ import types
 import pytest
 import torch
 
+from r2omni_b200 import build
 from r2omni_b200.sspa import executor as X
 from r2omni_b200.sspa.cache import PackedArenas
 
@@ -61,3 +62,10 @@ def test_native_step_follows_a_renewed_view_whoever_sees_it_first(prepared, betw
     assert len(made) == 2 and used[-1][0] is made[1], "launched with the addresses of the old view"
     ex(query)
     assert len(made) == 2
+
+
+def test_host_module_of_another_torch_or_python_is_stale(monkeypatch):
+    build.build_library()
+    assert not build.host_stale()
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".other")
+    assert build.host_stale()
