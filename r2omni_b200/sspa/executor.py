@@ -234,15 +234,16 @@ class SplitKExecutor:
             raise ValueError("step_host supports bf16 caches")
         nq, nkv = a.batch * self.num_query_heads * 128, a.batch * a.num_kv_heads * 128
         need = nq + (2 * nkv if append_indices is not None else 0)
-        if self._host_pair is not None and host_in is self._host_pair[0] and host_out is self._host_pair[1] \
-                and need == self._host_pair[2]:
-            pass   # the same buffers as in the last call: already checked
+        seen = self._host_pair
+        if seen is not None and host_in is seen[0] and host_out is seen[1] and seen[2:] == (
+                need, host_in.data_ptr(), host_out.data_ptr(), host_in.numel(), host_out.numel()):
+            pass   # the same tensors over the same memory as in the last call: already checked
         elif (host_in.device.type != "cpu" or host_out.device.type != "cpu" or host_in.dtype != a.dtype
                 or host_out.dtype != a.dtype or not host_in.is_contiguous() or not host_out.is_contiguous()
                 or host_in.numel() < need or host_out.numel() != nq):
             raise ValueError("host buffers do not match the prepared split-K executor")
         else:
-            self._host_pair = (host_in, host_out, need, host_in.data_ptr(), host_out.data_ptr())
+            self._host_pair = (host_in, host_out, need, host_in.data_ptr(), host_out.data_ptr(), host_in.numel(), host_out.numel())
         if append_indices is None and a.n_fp + a.n_i4 + a.i2_active + a.recent_len == 0:
             raise ValueError("four-quadrant cache has no surviving tokens")
         ap = None

@@ -64,6 +64,24 @@ def test_native_step_follows_a_renewed_view_whoever_sees_it_first(prepared, betw
     assert len(made) == 2
 
 
+def test_host_step_takes_the_addresses_its_tensors_have_now(prepared):
+    ex, _, _ = prepared
+    calls = []
+    ex._decode_host = lambda *args: calls.append(args) or 0
+    host_in, host_out = torch.zeros(256, dtype=torch.bfloat16), torch.zeros(1, 2, 128, dtype=torch.bfloat16)
+    ex.step_host(host_in, host_out)
+    ex.step_host(host_in, host_out)
+    moved_in, moved_out = torch.zeros(512, dtype=torch.bfloat16), torch.zeros(1, 2, 128, dtype=torch.bfloat16)
+    host_in.set_(moved_in)
+    host_out.set_(moved_out)
+    ex.step_host(host_in, host_out)
+    assert [c[2] for c in calls[1:]] == [calls[0][2], moved_in.data_ptr()]
+    assert [c[8] for c in calls[1:]] == [calls[0][8], moved_out.data_ptr()]
+    host_out.resize_(1, 2, 64)
+    with pytest.raises(ValueError):
+        ex.step_host(host_in, host_out)
+
+
 def test_host_module_of_another_torch_or_python_is_stale(monkeypatch):
     build.build_library()
     assert not build.host_stale()
