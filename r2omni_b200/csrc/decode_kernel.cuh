@@ -62,13 +62,6 @@ __device__ __forceinline__ Tile tile_of(const DecodeParams& p, int u) {
   return t;
 }
 
-// Residual tiles without rows are left out, except the first one of a CTA's range [u0, ..): producer and consumers each read
-// recent_len, the last head of the request to finish raises it, and only a tile that the consumers wait for orders the
-// producer's read before their arrival.  A read behind the raise would produce a tile that nobody consumes.
-__device__ __forceinline__ bool kept_residual_tile(const DecodeParams& p, int u, int u0, int win, int rlen) {
-  return win < rlen || u == max(u0, p.nF + p.n4 + p.n2);
-}
-
 // The unit range [u0,u1) of (request,kv head) `bh` inside a CTA's cost interval [c0, c1).
 __device__ __forceinline__ void unit_range(const DecodeParams& p, const CostPos& c0, const CostPos& c1, int bh, int& u0, int& u1) {
   const uint32_t lo = bh == c0.bh ? c0.r : 0u;
@@ -326,9 +319,8 @@ __device__ __forceinline__ void store_row(float* slot, int hh, int sub, float mx
 }
 
 // Every CTA of (b, h) has arrived, so none of them reads recent_len[b] any more: its consumers have read it before, and
-// its producer before the first residual tile of the CTA's range, which the consumers wait for (kept_residual_tile).
-// One thread outside the merge workers
-// counts the head in; the last head of the request moves the ring metadata; another warp writes the new rows.
+// its producer before a tile that they wait for.  One thread outside the merge workers counts the head in; the last head of
+// the request moves the ring metadata; another warp writes the new rows.
 static_assert(kNW >= 6, "warps 4 and 5 carry the request counter and the appended rows");
 __device__ __forceinline__ void commit_append(const DecodeParams& p, int b, int h, int rlen0) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -682,12 +674,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
       for (int u = u0; u < u1; ++u) {
         const Tile tl = tile_of(p, u);
         if (tl.pool == 3) {
+          // Tiles without rows are left out, except the first one of a CTA's range (it brings rows that nobody counts):
+          // producer and consumers each read recent_len, the last head of the request to finish raises it, and only a tile
+          // that the consumers wait for orders this read before their arrival.  Behind the raise it could produce a tile that
+          // nobody consumes.  A cluster needs nothing of the kind: its barrier waits for every thread that has not exited,
+          // the producer's among them.
+          bool first = false;
           if (rlen < 0) {
+            first = true;
             grid_dependency_wait();   // the ring and its length belong to the previous step until it has completed
             rlen = *reinterpret_cast<const int*>((const uint8_t*)p.v.recent_len + (size_t)b * p.v.recent_len_bstride) +
                    (has_append ? 1 : 0);
           }
-          if (!kept_residual_tile(p, u, u0, tl.win, rlen)) continue;
+          if (tl.win >= rlen && (CLUSTER || !first)) continue;
         }
         if (!mbar_wait_relaxed(&empty_bar[stage], phase ^ 1u)) {
           if (lane == 0) atomicExch(p.err, R2K_ERR_DEVICE_TIMEOUT);
@@ -697,9 +696,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
         uint8_t* sb = stages + stage * kStageBytes;
         const bool full = tl.pool < 3 && tl.lo == 0 && tl.hi == (tl.pool == 0 ? kTF : kTQ) &&
                           (tl.pool == 0 ? p.fp_tma != 0 : tl.pool == 1 ? src.fast1 : src.fast2);
-        if (tl.pool == 3 && tl.win >= rlen) {
-          if (lane == 0) mbar_arrive(&full_bar[stage]);   // no rows: the consumers only wait for it
-        } else if (full) {
+        if (full) {
           if (lane == 0) produce_full_tile(p, src, tl.pool, tl.win, b, h, sb, &full_bar[stage]);
         } else {
           produce_tile(p, tl, b, h, sb, &full_bar[stage], lane);
@@ -766,10 +763,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
     // residual window: kTR-token tiles, 16 tokens per warp; the lower half of the warps takes even tiles and the
     // upper half odd ones, so two tiles (the whole 128-token window) are in work at once
     set_units(st, 0);
-    for (int u = max(u0, p.nF + p.n4 + p.n2); u < u1; ++u) {
+    const int first_residual = max(u0, p.nF + p.n4 + p.n2);
+    for (int u = first_residual; u < u1; ++u) {
       const int ur = u - p.nF - p.n4 - p.n2;
       const int win = ur * kTR;
-      if (!kept_residual_tile(p, u, u0, win, rlen)) continue;
+      if (win >= rlen && (CLUSTER || u != first_residual)) continue;   // as the producer does
       if (alive && !mbar_wait(&full_bar[stage], phase)) {
         if (lane == 0) atomicExch(p.err, R2K_ERR_DEVICE_TIMEOUT);
         alive = false;
