@@ -127,3 +127,36 @@ def test_outputs_given_as_any_iterable():
     outs = [torch.empty_like(t) for t in (qd, kd, kd)]
     got = R.qwen_qkv_prologue(*rows, cd, sd, (16, 24, 24), output=iter(outs))
     assert all(a is b for a, b in zip(got, outs)) and torch.equal(outs[0], want[0]) and torch.equal(outs[2], kd)
+
+
+# Long prefills: a warp walks several heads with its tokens' table rows kept and the next head's rows in flight.  On 148 SMs
+# walks of 2 (18 heads), 4 (18 heads: a ragged last group), 7 (32 heads, ragged) and 8 (65601 heads of one token)
+@pytest.mark.parametrize("batch,hq,hkv,tokens,dtype,hadamard", [
+    (1, 16, 2, 4099, torch.bfloat16, False), (2, 16, 2, 4101, torch.float16, True), (1, 28, 4, 7001, torch.bfloat16, True),
+    (1, 65600, 1, 1, torch.bfloat16, True)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_warps_that_walk_several_heads(batch, hq, hkv, tokens, dtype, hadamard, in_place):
+    q, k, cos, sin = _inputs(batch, hq, hkv, tokens, dtype, dtype, seed=tokens + hq)
+    want_q, want_k = O.qk_mrope(q, k, cos, sin, (16, 24, 24), hadamard)
+    qd, kd = q.cuda(), k.cuda()
+    got_q, got_k = R.qwen_qk_mrope(qd, kd, cos.cuda(), sin.cuda(), (16, 24, 24), apply_hadamard=hadamard,
+                                   output=(qd, kd) if in_place else None)
+    assert torch.equal(got_q.cpu().view(torch.int16), want_q.view(torch.int16))
+    assert torch.equal(got_k.cpu().view(torch.int16), want_k.view(torch.int16))
+
+
+@pytest.mark.parametrize("value_hadamard", [False, True])
+def test_prologue_walks_from_keys_into_values(value_hadamard):
+    batch, hq, hkv = 6201, 16, 4   # walks of five of the 24 heads on 148 SMs
+    g = torch.Generator().manual_seed(5)
+    fused = torch.randn(batch, 1, (hq + 2 * hkv) * 128, generator=g).to(torch.bfloat16)
+    q, k, v = fused.split([hq * 128, hkv * 128, hkv * 128], dim=2)
+    _, _, cos, sin = _inputs(batch, 1, 1, 1, torch.bfloat16, torch.bfloat16, seed=6)
+    d = fused.cuda()
+    got = R.qwen_qkv_prologue(*d.split([hq * 128, hkv * 128, hkv * 128], dim=2), cos.cuda(), sin.cuda(), (16, 24, 24),
+                              key_hadamard=True, value_hadamard=value_hadamard)
+    rows = lambda t, h: t.reshape(batch, h, 1, 128)  # noqa: E731
+    want_q, want_k = O.qk_mrope(rows(q, hq), rows(k, hkv), cos, sin, (16, 24, 24), True)
+    want_v = O.fwht128(rows(v, hkv).float()).to(torch.bfloat16) if value_hadamard else rows(v, hkv)
+    for a, b in zip(got, (want_q, want_k, want_v)):
+        assert torch.equal(a.cpu().view(torch.int16), b.contiguous().view(torch.int16))
