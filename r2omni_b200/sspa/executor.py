@@ -235,15 +235,15 @@ class SplitKExecutor:
         nq, nkv = a.batch * self.num_query_heads * 128, a.batch * a.num_kv_heads * 128
         need = nq + (2 * nkv if append_indices is not None else 0)
         seen = self._host_pair
-        if seen is not None and host_in is seen[0] and host_out is seen[1] and seen[2:] == (
-                need, host_in.data_ptr(), host_out.data_ptr(), host_in.numel(), host_out.numel()):
+        if (seen is not None and host_in is seen[0] and host_out is seen[1] and need == seen[2] and host_in.data_ptr() == seen[3]
+                and host_out.data_ptr() == seen[4] and host_in.numel() >= need and host_out.numel() == nq):
             pass   # the same tensors over the same memory as in the last call: already checked
         elif (host_in.device.type != "cpu" or host_out.device.type != "cpu" or host_in.dtype != a.dtype
                 or host_out.dtype != a.dtype or not host_in.is_contiguous() or not host_out.is_contiguous()
                 or host_in.numel() < need or host_out.numel() != nq):
             raise ValueError("host buffers do not match the prepared split-K executor")
         else:
-            self._host_pair = (host_in, host_out, need, host_in.data_ptr(), host_out.data_ptr(), host_in.numel(), host_out.numel())
+            self._host_pair = (host_in, host_out, need, host_in.data_ptr(), host_out.data_ptr())
         if append_indices is None and a.n_fp + a.n_i4 + a.i2_active + a.recent_len == 0:
             raise ValueError("four-quadrant cache has no surviving tokens")
         ap = None
