@@ -173,7 +173,8 @@ struct LaneOffsets {
 // accumulation is the only rounding.  Codes minus zero points are fed as signed fp16 subnormals (AND, HSUB2).
 // The four 32-channel steps are the outer loop: Q' and the zero points of a step live for that step only (12 registers
 // instead of 48) and both tiles' four MMA chains run side by side.  Same sums in the same order as with the tiles
-// outermost; four 8 x 32768-token layers 128.5 -> 120.9 us, 16 x 4 heads x 65536 tokens 178.6 -> 167.7 us.
+// outermost; four 8 x 32768-token layers 128.5 -> 120.9 us and 16 x 4 heads x 65536 tokens 178.6 -> 167.7 us in a loop over the
+// same inputs when it was made, 2 to 3 % more since value metadata may lie at any alignment (copy_meta).
 __device__ __forceinline__ void qk_int4(uint32_t sb, const LaneOffsets& o, const uint32_t (&qh)[16], float alpha,
                                         float (&s)[2][4]) {
   uint32_t w[4][4];   // key words of row 16 j + 8 e (index 2 j + e), one per channel step

@@ -97,8 +97,7 @@ __device__ __forceinline__ void zero_piece(uint8_t* dst, int bytes, int lane) {
 // boundaries (every head but the first behind an odd INT4 pool, every pool behind an odd one).  The window's row 0 is
 // placed `src & 15` bytes into its region, and whole granules are copied: none of them lies outside the memory that holds the
 // rows.  Neighbours' rows that come along are masked by the consumers.  With plain loads for such tiles, one byte per
-// lane and step, a launch of 200003 tokens x 4 heads took 272 us,
-// now 45.5.
+// lane and step, a launch of 200003 tokens x 4 heads took 272 us, now 45.5.
 __device__ __forceinline__ uint32_t meta_shift(const uint8_t* row0) { return (uint32_t)(uintptr_t)row0 & 15u; }
 __device__ __forceinline__ uint32_t copy_meta(uint8_t* region, const uint8_t* row0, int first, int bytes, uint64_t* bar) {
   const uint8_t* src = row0 + first;
@@ -148,7 +147,8 @@ __device__ __forceinline__ void produce_tile(const DecodeParams& p, const Tile& 
     const size_t meta = (size_t)h * (p.g.k_capacity >> p.kblock_shift) + blk0;
     copy_piece(stage + off_ks(tl.pool), (const uint8_t*)v.k_scale + (size_t)b * v.k_scale_bstride + meta * 256, nblk * 256, bar, lane, tx);
     copy_piece(stage + off_kz(tl.pool), v.k_zero + (size_t)b * v.k_zero_bstride + meta * 128, nblk * 128, bar, lane, tx);
-    // values: only rows of this pool; rows of the window outside it are cleared
+    // values: only rows of this pool.  bf16 rows of the window outside it are cleared (0 * NaN); packed ones are whatever the
+    // stage held, any bits of which are finite codes, under scales that the consumers replace by zero
     uint8_t* vreg = stage + kOffV;
     if (tl.pool == 0) {
       const size_t row = (size_t)h * p.g.fp_capacity + (tl.win + tl.lo - p.g.k_off_fp);
@@ -199,7 +199,7 @@ __device__ __forceinline__ TileSources tile_sources(const DecodeParams& p, int b
   s.s1 = (const uint8_t*)v.i4_scale + (int64_t)b * v.i4_scale_bstride + r1 * 4;
   s.s2 = (const uint8_t*)v.i2_scale + (int64_t)b * v.i2_scale_bstride + r2 * p.groups2 * 2;
   s.z2 = v.i2_zero + (int64_t)b * v.i2_zero_bstride + r2 * p.groups2;
-  // full tiles start at multiples of 64 rows, so base alignment decides everything
+  // full tiles start at multiples of kTQ rows, so base alignment decides everything
   s.fast1 = ((uintptr_t)s.v1 & 15) == 0;
   s.fast2 = ((uintptr_t)s.v2 & 15) == 0;
   return s;

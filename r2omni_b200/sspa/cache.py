@@ -10,7 +10,6 @@ reference-shaped objects (``ThreePrecisionCache``, ``PrecisionPool``,
 """
 from __future__ import annotations
 
-import ctypes as C
 from dataclasses import dataclass, field
 from enum import IntEnum
 from typing import Literal
@@ -48,10 +47,6 @@ class LayerCompressionPlan:
     page_offsets: torch.Tensor
     page_lengths: torch.Tensor
     page_classes: torch.Tensor
-
-
-def _ceil_to(value: int, multiple: int) -> int:
-    return -(-int(value) // int(multiple)) * int(multiple)
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -552,7 +547,7 @@ def precision_cache_active_storage_breakdown(cache: ThreePrecisionCache) -> dict
 # --------------------------------------------------------------------------- #
 def tier_sorted_tokens(plan: LayerCompressionPlan):
     """Stable reorder of pages into (bf16-V, INT4-V, INT2-V, evicted) token lists
-    (precision_pool.py:611-669), computed on the host from the small page table."""
+    (precision_pool.py:611-669): the order in which the native build lays a cache out, one list entry per token."""
     classes = plan.page_classes.detach().cpu().long()
     offsets = plan.page_offsets.detach().cpu().long()
     lengths = plan.page_lengths.detach().cpu().long()
@@ -595,7 +590,11 @@ def build_three_precision_cache(
 ) -> ThreePrecisionCache:
     """Stable page reorder into contiguous bf16/INT4/INT2 value pools over one
     INT4 key arena, plus the residual ring (precision_pool.py:787-984), packed on
-    the device by this library's kernels."""
+    the device by this library's kernels, in one launch.
+
+    The cache's tensors share one allocation: it is freed when the last of them is, and saving one of them with
+    ``torch.save`` writes the whole block unless it is cloned first.  Values may be of the other 16-bit type than the
+    keys; the cache takes the keys' type.  Refused while a CUDA graph is captured (the page table is uploaded)."""
     if key.shape != value.shape or key.ndim != 3:
         raise ValueError("key/value must be logical [Hkv,S,D]")
     if int(key.shape[1]) != int(plan.logical_positions.numel()):
