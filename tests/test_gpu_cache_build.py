@@ -218,3 +218,17 @@ def test_pages_without_tokens_may_start_anywhere():
     a = R.build_three_precision_cache(key, key, plan, page_size=16).arenas
     b = R.build_three_precision_cache(key, key, _plan([2, 1, 5], [16, 0, 16]), page_size=16).arenas
     assert torch.equal(a.k_packed, b.k_packed) and torch.equal(a.i2_packed, b.i2_packed) and torch.equal(a.i4_packed, b.i4_packed)
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_build_is_refused_while_a_graph_is_captured(mode):
+    """The page table is uploaded from a block that the call gives back: a replay would read whatever lies there then."""
+    plan = _plan([2, 1], [16, 16])
+    key = torch.zeros(1, 32, 128, dtype=torch.bfloat16, device="cuda")
+    R.build_three_precision_cache(key, key, plan, page_size=16)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), capture_error_mode=mode):
+            R.build_three_precision_cache(key, key, plan, page_size=16)
+    torch.cuda.synchronize()
+    assert int(R.build_three_precision_cache(key, key, plan, page_size=16).arenas.recent_len_device) == 0
