@@ -285,16 +285,16 @@ __device__ __forceinline__ void merge_rows(const float* base, int count, int own
   }
 }
 
-// The same for the kCluster partials of a cluster's CTAs, read out of their shared memory (`slot`: this CTA's own).
-__device__ __forceinline__ void merge_cluster_rows(const float* slot, int hh, int sub, float& mx, float& lsum, float (&acc)[8]) {
-  float4 ml[kCluster], va[kCluster], vb[kCluster];
-  const uint32_t row = smem_u32(slot + hh * kRowFloats);
+// The same for the kCluster rows of one head that a cluster's CTAs have put into this CTA's inbox.
+__device__ __forceinline__ void merge_cluster_rows(const float* inbox, int sub, float& mx, float& lsum, float (&acc)[8]) {
+  float2 ml[kCluster];
+  float4 va[kCluster], vb[kCluster];
 #pragma unroll
   for (int k = 0; k < kCluster; ++k) {
-    const uint32_t a = cluster_map(row, (uint32_t)k);
-    ml[k] = ld_cluster_f4(a);
-    va[k] = ld_cluster_f4(a + 16 + 32 * sub);
-    vb[k] = ld_cluster_f4(a + 32 + 32 * sub);
+    const float* row = inbox + k * kRowFloats;
+    ml[k] = *reinterpret_cast<const float2*>(row);
+    va[k] = *reinterpret_cast<const float4*>(row + 4 + 8 * sub);
+    vb[k] = *reinterpret_cast<const float4*>(row + 8 + 8 * sub);
   }
   mx = -INFINITY;
 #pragma unroll
@@ -318,27 +318,23 @@ __device__ __forceinline__ void store_row(float* slot, int hh, int sub, float mx
   if (sub == 0) __stcg(reinterpret_cast<float2*>(orow), make_float2(mx, lsum));
 }
 
-// Every CTA of (b, h) has arrived, so none of them reads recent_len[b] any more: its consumers have read it before, and
-// its producer before a tile that they wait for.  One thread outside the merge workers counts the head in; the last head of
-// the request moves the ring metadata; another warp writes the new rows.
+// Every CTA of (b, h) has read recent_len[b]: its consumers, and its producer before a tile that they wait for (a cluster's
+// producer does not read it).  The loads have returned, so no fence is wanted in front of the count.  One thread outside the
+// merge workers counts the head in; the last head of the request moves the ring metadata; another warp writes the new rows.
 static_assert(kNW >= 6, "warps 4 and 5 carry the request counter and the appended rows");
 __device__ __forceinline__ void commit_append(const DecodeParams& p, int b, int h, int rlen0) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool has_append = p.app_k != nullptr;
-  if (threadIdx.x == 128) {
-    __threadfence();
-    const int done = atomicAdd(&p.req_counter[b], 1);
-    if (done == p.g.num_kv_heads - 1) {
-      p.req_counter[b] = 0;
-      if (has_append) {
-        const int64_t gi = p.app_idx ? p.app_idx[2 * b] : p.app_global;
-        const int64_t lp = p.app_idx ? p.app_idx[2 * b + 1] : p.app_logical;
-        *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_global + (size_t)b * p.v.recent_global_bstride + 8 * (size_t)rlen0) = gi;
-        *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_logical + (size_t)b * p.v.recent_logical_bstride + 8 * (size_t)rlen0) = lp;
-        *reinterpret_cast<int*>((uint8_t*)p.v.recent_len + (size_t)b * p.v.recent_len_bstride) = rlen0 + 1;
-        *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_page_lengths + (size_t)b * p.v.recent_page_lengths_bstride +
-                                    8 * (size_t)(rlen0 / p.g.page_size)) = rlen0 % p.g.page_size + 1;
-      }
+  if (threadIdx.x == 128 && atomicAdd(&p.req_counter[b], 1) == p.g.num_kv_heads - 1) {
+    p.req_counter[b] = 0;
+    if (has_append) {
+      const int64_t gi = p.app_idx ? p.app_idx[2 * b] : p.app_global;
+      const int64_t lp = p.app_idx ? p.app_idx[2 * b + 1] : p.app_logical;
+      *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_global + (size_t)b * p.v.recent_global_bstride + 8 * (size_t)rlen0) = gi;
+      *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_logical + (size_t)b * p.v.recent_logical_bstride + 8 * (size_t)rlen0) = lp;
+      *reinterpret_cast<int*>((uint8_t*)p.v.recent_len + (size_t)b * p.v.recent_len_bstride) = rlen0 + 1;
+      *reinterpret_cast<int64_t*>((uint8_t*)p.v.recent_page_lengths + (size_t)b * p.v.recent_page_lengths_bstride +
+                                  8 * (size_t)(rlen0 / p.g.page_size)) = rlen0 % p.g.page_size + 1;
     }
   }
   if (has_append && warp == 5) {  // ring row rlen0 of head h
@@ -630,8 +626,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* stages = smem;
   float* scratch = reinterpret_cast<float*>(smem + kStages * kStageBytes);
-  float* cluster_slot = scratch + kNW * kSlotFloats;   // this CTA's partial, where the cluster's other CTAs read it
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(cluster_slot + (CLUSTER ? kSlotFloats : 0));
+  float* inbox = scratch + kNW * kSlotFloats;   // a cluster's rows of the head that this CTA merges, one per rank
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(inbox + (CLUSTER ? kSlotFloats : 0));
   uint64_t* empty_bar = full_bar + kStages;
   uint32_t* const_block = reinterpret_cast<uint32_t*>(empty_bar + kStages);   // see PoolConsts
   int* flags = reinterpret_cast<int*>(const_block) + kConstBytes / 4;  // [0] last-arriver flag
@@ -665,6 +661,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
   if (warp == kNW) {
     // ------------------------------ producer ------------------------------
     bool alive = true;
+    if (CLUSTER) cluster_arrive();   // as the consumers' first arrival: this warp has nothing to read before it
     for (int bh = bh_lo; bh <= bh_hi && alive; ++bh) {
       const int b = bh / p.g.num_kv_heads, h = bh - b * p.g.num_kv_heads;
       int u0, u1;
@@ -673,12 +670,15 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
       const TileSources src = tile_sources(p, b, h);
       for (int u = u0; u < u1; ++u) {
         const Tile tl = tile_of(p, u);
-        if (tl.pool == 3) {
+        if (CLUSTER && tl.pool == 3) {
+          // The window belongs to the previous step until that has completed.  Its tiles come whole, whatever its length: a load of
+          // the length in front of them is another trip to memory on the way of a short launch.
+          grid_dependency_wait();
+        } else if (tl.pool == 3) {
           // Tiles without rows are left out, except the first one of a CTA's range (it brings rows that nobody counts):
           // producer and consumers each read recent_len, the last head of the request to finish raises it, and only a tile
           // that the consumers wait for orders this read before their arrival.  Behind the raise it could produce a tile that
-          // nobody consumes.  A cluster needs nothing of the kind: its barrier waits for every thread that has not exited,
-          // the producer's among them.
+          // nobody consumes.
           bool first = false;
           if (rlen < 0) {
             first = true;
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
             rlen = *reinterpret_cast<const int*>((const uint8_t*)p.v.recent_len + (size_t)b * p.v.recent_len_bstride) +
                    (has_append ? 1 : 0);
           }
-          if (tl.win >= rlen && (CLUSTER || !first)) continue;
+          if (tl.win >= rlen && !first) continue;
         }
         if (!mbar_wait_relaxed(&empty_bar[stage], phase ^ 1u)) {
           if (lane == 0) atomicExch(p.err, R2K_ERR_DEVICE_TIMEOUT);
@@ -703,6 +703,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
         }
         if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
+    }
+    if (CLUSTER) {   // both of the cluster's barriers in full: a thread that left between its arrival and its wait would count twice
+      cluster_wait();
+      cluster_arrive();
+      cluster_wait();
     }
     return;
   }
@@ -767,7 +772,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
     for (int u = first_residual; u < u1; ++u) {
       const int ur = u - p.nF - p.n4 - p.n2;
       const int win = ur * kTR;
-      if (win >= rlen && (CLUSTER || u != first_residual)) continue;   // as the producer does
+      if (!CLUSTER && win >= rlen && u != first_residual) continue;   // as the producer does
       if (alive && !mbar_wait(&full_bar[stage], phase)) {
         if (lane == 0) atomicExch(p.err, R2K_ERR_DEVICE_TIMEOUT);
         alive = false;
@@ -786,8 +791,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
                   __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_k + off));
               *reinterpret_cast<uint2*>(sbp + kOffV + kOffRecentV + (r0 + app_row) * 256 + 8 * lane) =
                   __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_v + off));
-              __syncwarp();
             }
+            for (int i = hi; CLUSTER && i < 16; ++i)   // rows behind the window's last one: 0 * NaN must not reach a value
+              *reinterpret_cast<uint2*>(sbp + kOffV + kOffRecentV + (r0 + i) * 256 + 8 * lane) = make_uint2(0u, 0u);
+            __syncwarp();
             const int t0 = 2 * t + (t & 1), t1 = 2 * t + 1 - (t & 1);
             float s[1][4];
             qk_fp<BF16>(sb + kOffV + (r0 + pg) * 256 + 64 * t, qrow, t, p.qscale, s[0]);
@@ -797,10 +804,17 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
                                s[0]);
           }
         }
+        if (CLUSTER) fence_async_shared();   // the plain stores above, before the producer's next copies into the stage
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty_bar[stage]);
       }
       if (++stage == kStages) { stage = 0; phase ^= 1u; }
+    }
+
+    // The consumers' first arrival at the cluster's barrier: each has read recent_len.
+    if (CLUSTER) {
+      wait_for_value(rlen0);
+      cluster_arrive();
     }
 
     // ---- this CTA's partial for (b, h): merge the eight warps through shared memory ----
@@ -846,33 +860,36 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
       own_m = mx; own_l = lsum;
       own_acc[0] = a0.x; own_acc[1] = a0.y; own_acc[2] = a0.z; own_acc[3] = a0.w;
       own_acc[4] = a1.x; own_acc[5] = a1.y; own_acc[6] = a1.z; own_acc[7] = a1.w;
-      if (CLUSTER) {
-        float* orow = cluster_slot + hh * kRowFloats;
-        *reinterpret_cast<float4*>(orow + 4 + 8 * sub) = a0;
-        *reinterpret_cast<float4*>(orow + 8 + 8 * sub) = a1;
-        if (sub == 0) *reinterpret_cast<float4*>(orow) = make_float4(mx, lsum, 0.f, 0.f);
+      if (CLUSTER) {   // head hh's row goes to the CTA of rank hh
+        cluster_wait();   // every CTA of the cluster runs: its inbox is there
+        const uint32_t row = cluster_map(smem_u32(inbox + cluster_rank() * kRowFloats), (uint32_t)hh);
+        st_cluster_f4(row + 16 + 32 * sub, a0);
+        st_cluster_f4(row + 32 + 32 * sub, a1);
+        if (sub == 0) st_cluster_f4(row, make_float4(mx, lsum, 0.f, 0.f));
       } else {
         store_row(slot, hh, sub, own_m, own_l, own_acc);
       }
     }
     if (CLUSTER) {
       // ---- one exact merge through distributed shared memory: the CTA of rank r merges head r of the group ----
-      // Two cluster barriers and one round of remote loads where the path below pays a store, a fence, a ticket and a
-      // round of loads through L2.  A cluster's CTAs hold one (request, kv head) each, so all of them come here once.
+      // A round of remote stores and one cluster barrier where the path below pays a store, a fence, a ticket and a round of loads
+      // through L2, and nobody's shared memory is touched by others behind that barrier.  The append goes ahead beside the merge.
+      // (Partials read out of the other CTAs, a barrier in front of the exit, the append behind the merge and the length read in front
+      // of the window's copies: 239.9 us for 36 launches of 701 tokens x 2 heads, 316.9 of 4096; so 224.5 and 309.7.)  A cluster's
+      // CTAs hold one (request, kv head) each, so all of them come here once.
+      const int rank = (int)cluster_rank();
+      if (!worker) {
+        cluster_wait();
+        if (rank == 0) commit_append(p, b, h, rlen0);
+      }
       cluster_arrive();
       cluster_wait();
-      const int rank = (int)cluster_rank();
       if (warp == 0) {   // both halves of the warp do the same; the lower one stores
         const int sub = lane & 15;
         float mx, lsum, acc[8];
-        merge_cluster_rows(cluster_slot, rank, sub, mx, lsum, acc);
+        merge_cluster_rows(inbox, sub, mx, lsum, acc);
         write_output<BF16>(p, (size_t)b * p.g.num_q_heads + h * p.gqa + rank, rank < p.gqa && lane < 16, sub, mx, lsum, acc);
-      } else if (rank == 0) {
-        commit_append(p, b, h, rlen0);
       }
-      __syncwarp();
-      cluster_arrive();   // nobody leaves while its partial may still be read
-      cluster_wait();
       return;
     }
     // ---- two-level exact merge: groups of kMergeGroup partials, then the group results ----

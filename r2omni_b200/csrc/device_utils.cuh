@@ -150,6 +150,9 @@ __device__ __forceinline__ void tensor_g2s_4d(void* dst_smem, const void* tmap, 
       : "memory");
 }
 
+// Orders this thread's plain accesses to shared memory before bulk copies that are issued behind it.
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+
 // System-scope flag traffic between GPUs (peer memory over NVLink).
 __device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t* p) {
   uint32_t v;
@@ -193,16 +196,18 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
   return r;
 }
-// Address of `a` (this CTA's shared memory) in the CTA of rank `rank`, and a 16-byte load from there.
+// Holds the thread until `x` is there: an instruction that reads it and does nothing, whatever its value.
+__device__ __forceinline__ void wait_for_value(int x) {
+  asm volatile("{\n.reg .pred p;\nsetp.eq.s32 p, %0, -2147483648;\n@p nanosleep.u32 0;\n}\n" ::"r"(x));
+}
+// Address of `a` (this CTA's shared memory) in the CTA of rank `rank`, and a 16-byte store to there.
 __device__ __forceinline__ uint32_t cluster_map(uint32_t a, uint32_t rank) {
   uint32_t d;
   asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(d) : "r"(a), "r"(rank));
   return d;
 }
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
+__device__ __forceinline__ void st_cluster_f4(uint32_t a, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 // Programmatic dependent launch.  launch_dependents lets the next kernel of the stream (when it was launched with

@@ -1,0 +1,42 @@
+"""Small caches (one cluster of CTAs per head) fetch the residual window whole, whatever its length: rows behind the last one must
+not reach the result, whatever they hold."""
+import pytest
+import torch
+
+from gpu_helpers import make_executor
+from test_gpu_decode import both_caches, seeded_classes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("length", [0, 1, 15, 16, 17, 63, 64, 65, 80, 127, 128])
+def test_rows_behind_the_window_do_not_count(length, dtype):
+    pages, heads = 9, 3
+    _, cache, new_k, new_v, queries = both_caches(7, hq=5 * heads, hkv=heads, tokens=pages * 32, page=32,
+                                                  classes=seeded_classes(pages, 3), appends=128, dtype=dtype, append_capacity=256)
+    ex = make_executor(cache, 5 * heads)
+    a, q = cache.arenas, queries[0].cuda()
+    rows_k, rows_v = (t.transpose(0, 1).unsqueeze(0).cuda() for t in (new_k, new_v))   # [1, heads, 128, 128]
+
+    def fill(rest):
+        a.recent_k.fill_(rest)
+        a.recent_v.fill_(rest)
+        a.recent_k[:, :, :length], a.recent_v[:, :, :length] = rows_k[:, :, :length], rows_v[:, :, :length]
+        a.recent_len_device.fill_(length)
+        a.recent_len = length
+
+    fill(0.0)
+    want = ex.decode_f32(q).clone()
+    fill(float("nan"))
+    assert torch.isfinite(want).all() and torch.equal(ex.decode_f32(q), want)
+    if length < 128:   # the appended row takes the place of the first of them
+        outs = []
+        for rest in (0.0, float("nan")):
+            fill(rest)
+            step = (new_k[length].unsqueeze(0).cuda().contiguous(), new_v[length].unsqueeze(0).cuda().contiguous(), 500, 500)
+            outs.append(ex(q, append=step).clone())
+            assert int(a.recent_len_device) == length + 1
+            assert torch.equal(a.recent_k[:, :, length], rows_k[:, :, length]) and torch.equal(a.recent_v[:, :, length], rows_v[:, :, length])
+        assert torch.isfinite(outs[0].float()).all() and torch.equal(outs[0], outs[1])
+    assert ex.device_status() == 0
