@@ -379,6 +379,7 @@ __device__ __forceinline__ void split_row(const Row16& r, bool hadamard, float (
 // In place when out == in.
 template <bool BF16>
 __global__ void __launch_bounds__(128) fwht128_kernel(const uint16_t* in, uint16_t* out, int64_t rows, bool wide) {
+  grid_dependency_wait();   // launched with programmatic stream serialization: only the way here overlaps the kernel in front
   const int64_t row = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4 + ((threadIdx.x & 31) >> 3);
   const int s = threadIdx.x & 7;
   const bool valid = row < rows;   // every lane takes part in the shuffles

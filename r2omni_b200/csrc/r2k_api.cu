@@ -717,10 +717,13 @@ int r2k_merge_states(const float* states, int32_t num_states, int64_t state_stri
   if (states == nullptr || out == nullptr) return R2K_ERR_NULL;
   if (num_states < 1 || rows < 1 || (dtype != R2K_DTYPE_BF16 && dtype != R2K_DTYPE_FP16)) return R2K_ERR_GEOMETRY;
   if ((reinterpret_cast<uintptr_t>(states) & 7u) || (state_stride & 1) || !aligned16(out)) return R2K_ERR_ALIGNMENT;
-  merge_states_kernel<<<(rows + 3) / 4, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(states, num_states, state_stride, rows,
-                                                                                         dtype, out, flags);
+  DeviceInfo* dev;
+  const int rc = device_info(&dev);
+  if (rc) return rc;
+  const cudaError_t err = launch_behind(merge_states_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), reinterpret_cast<cudaStream_t>(stream),
+                                        dev->pdl, states, num_states, state_stride, rows, dtype, out, flags);
   ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
 }
 
 static int check_pack(const void* src, int32_t dtype, int32_t heads, int64_t src_rows, int64_t count, int64_t capacity,
@@ -858,12 +861,13 @@ int r2k_fwht128(const void* in, void* out, int32_t dtype, int64_t rows, void* st
   const unsigned grid = (unsigned)((rows + 15) / 16);
   const bool wide = aligned16(in) && aligned16(out);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == R2K_DTYPE_BF16)
-    fwht128_kernel<true><<<grid, 128, 0, st>>>(reinterpret_cast<const uint16_t*>(in), reinterpret_cast<uint16_t*>(out), rows, wide);
-  else
-    fwht128_kernel<false><<<grid, 128, 0, st>>>(reinterpret_cast<const uint16_t*>(in), reinterpret_cast<uint16_t*>(out), rows, wide);
+  DeviceInfo* dev;
+  const int rc = device_info(&dev);
+  if (rc) return rc;
+  const cudaError_t err = launch_behind(dtype == R2K_DTYPE_BF16 ? fwht128_kernel<true> : fwht128_kernel<false>, dim3(grid), dim3(128), st, dev->pdl,
+                                        reinterpret_cast<const uint16_t*>(in), reinterpret_cast<uint16_t*>(out), rows, wide);
   ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
 }
 
 int r2k_qk_mrope(const void* q, const void* k, void* q_out, void* k_out, int32_t dtype, int32_t batch, int32_t num_q_heads,

@@ -1,0 +1,47 @@
+"""Launches that come in while the kernel in front of them is still running (the state merge, the Hadamard transform): a chain of
+them without a synchronisation gives what the same calls give one at a time."""
+import pytest
+import torch
+
+import r2omni_b200 as R
+from gpu_helpers import make_executor
+from test_gpu_decode import both_caches, seeded_classes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("pages", [4, 700])   # a cluster per head, and the whole grid
+def test_state_and_merge_in_a_chain(pages):
+    _, cache, new_k, new_v, _ = both_caches(11, hq=16, hkv=2, tokens=pages * 32, page=32, classes=seeded_classes(pages, 3), appends=40,
+                                            append_capacity=256)
+    ex = R.SequenceShardedExecutor(make_executor(cache, 16))
+    queries = torch.randn(40, 1, 16, 128, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    k, v, a = new_k.cuda(), new_v.cuda(), cache.arenas
+
+    def steps(wait):
+        a.recent_len_device.zero_()
+        a.recent_len = 0
+        outs = []
+        for i in range(40):   # each step attends to the rows that the steps before it appended
+            out = ex(queries[i], append=(k[i:i + 1].contiguous(), v[i:i + 1].contiguous(), i, i))
+            a.recent_len = i + 1
+            outs.append(out.clone() if wait or i % 3 else out.float().to(out.dtype))
+            if wait:
+                torch.cuda.synchronize()
+        return torch.stack(outs)
+
+    want = steps(True)
+    assert torch.equal(steps(False), want) and int(a.recent_len_device) == 40
+
+
+@pytest.mark.parametrize("rows", [1, 15, 4096, 300000])
+def test_transforms_in_a_chain(rows):
+    x = torch.randn(rows, 128, generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda").to(torch.bfloat16)
+    want = x.clone()
+    for _ in range(6):
+        want = R.triton_fwht_128(want)
+        torch.cuda.synchronize()
+    got = x.clone()
+    for _ in range(6):
+        R.triton_fwht_128(got, output=got)   # in place: each reads what the one in front of it writes
+    assert torch.equal(got, want)
