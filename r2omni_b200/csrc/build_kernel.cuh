@@ -1,10 +1,14 @@
 // A whole packed cache from one layer's keys and values in one launch (r2k_build_cache).
 //
-// One CTA takes 128 arena rows of one head: four warps quantise the key blocks, 32 rows each, the other four the same
-// rows' values, each in the format of its pool.  Every key and value row is read once.  Further CTAs write the token
-// bookkeeping and set what lies behind the last used row.  Source rows come from the page table (a page's rows are
-// consecutive), so nothing per token is uploaded.  A build of 32768 tokens x 2 heads takes 56 us in all, host work included,
-// where four launches over token-index arrays, a fill per arena and an upload per index array took 1.35 ms.
+// One CTA takes 128 arena rows of one head, eight rows a warp: their keys first (the warps of a key block exchange their channels'
+// ranges), then their values, each in the format of its pool.  Every key and value row is read once.  Further CTAs write the
+// token bookkeeping and set what lies behind the last used row.  Source rows come from the page table (a page's rows are
+// consecutive), so nothing per token is uploaded.
+//
+// Bound by the IEEE divisions (one per key and per quantised value) and the way to them: page search, rows, range, divide.  With
+// 32 rows a warp, keys and values on different warps and one value row at a time, a CTA took 27 us from end to end, and the launch for
+// 32768 tokens x 2 heads 48 us; so 14 and 33.5 us (the rows' bytes alone take 7 us at the copy rate).  With all registers
+// (108 instead of 64, one CTA an SM) 37.5.
 #pragma once
 
 #include "pack_kernels.cuh"
@@ -12,7 +16,8 @@
 
 namespace r2k {
 
-constexpr int kBuildRows = 128, kBuildThreads = 256;
+constexpr int kBuildRows = 128, kBuildThreads = 512;
+constexpr int kWarpRows = kBuildRows / (kBuildThreads / 32);   // 8
 constexpr int kMaxFills = 13;
 constexpr int64_t kFillBytes = 16384;   // per CTA
 
@@ -46,35 +51,39 @@ __device__ __forceinline__ int page_of(const R2KBuild& b, int r) {
   return lo;
 }
 
-template <bool BF16>
-__device__ __forceinline__ void build_keys(const R2KBuild& b, int chunk, int head, const int* src_row, float (*range)[128][2]) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;   // warps 0-3: rows 32 warp ..
-  const uint16_t* src = reinterpret_cast<const uint16_t*>(b.key) + (int64_t)head * b.rows * 128 + 4 * lane;
-  uint2 w[32];
+// A warp's rows of one tensor, four channels a lane; a row behind the last token reads as zeros.
+__device__ __forceinline__ void load_rows(const void* base, int64_t rows, int head, const int* src_row, uint2 (&w)[kWarpRows]) {
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(base) + (int64_t)head * rows * 128 + 4 * (threadIdx.x & 31);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int s = src_row[32 * warp + i];
-    // a row behind the last token counts as zeros, which the range contains anyway
+  for (int i = 0; i < kWarpRows; ++i) {
+    const int s = src_row[i];
     w[i] = s >= 0 ? __ldcs(reinterpret_cast<const uint2*>(src + (int64_t)s * 128)) : make_uint2(0u, 0u);
   }
-  float lo[4], hi[4];
+}
+
+template <bool BF16>
+__device__ __forceinline__ void build_keys(const R2KBuild& b, int chunk, int head, const int* src_row, const uint2 (&w)[kWarpRows],
+                                           float4 (*range)[2][32]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float lo[4], hi[4];   // a range contains zero, so the zeros behind the last token change nothing
 #pragma unroll
   for (int e = 0; e < 4; ++e) lo[e] = hi[e] = 0.f;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
+  for (int i = 0; i < kWarpRows; ++i) {
     float x[4];
     unpack4<BF16>(w[i], x);
 #pragma unroll
     for (int e = 0; e < 4; ++e) { lo[e] = fminf(lo[e], x[e]); hi[e] = fmaxf(hi[e], x[e]); }
   }
-  if (b.k_block > 32) {   // a block spans two or four warps
-#pragma unroll
-    for (int e = 0; e < 4; ++e) { range[warp][4 * lane + e][0] = lo[e]; range[warp][4 * lane + e][1] = hi[e]; }
-    named_bar_sync(1, 128);
-    const int n = b.k_block / 32, first = warp / n * n;
-    for (int k = first; k < first + n; ++k)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { lo[e] = fminf(lo[e], range[k][4 * lane + e][0]); hi[e] = fmaxf(hi[e], range[k][4 * lane + e][1]); }
+  range[warp][0][lane] = make_float4(lo[0], lo[1], lo[2], lo[3]);
+  range[warp][1][lane] = make_float4(hi[0], hi[1], hi[2], hi[3]);
+  __syncthreads();
+  const int n = b.k_block / kWarpRows, first = warp / n * n;   // the warps of this block: 4, 8 or 16
+#pragma unroll 4
+  for (int k = first; k < first + n; ++k) {
+    const float4 l = range[k][0][lane], h = range[k][1][lane];
+    lo[0] = fminf(lo[0], l.x); lo[1] = fminf(lo[1], l.y); lo[2] = fminf(lo[2], l.z); lo[3] = fminf(lo[3], l.w);
+    hi[0] = fmaxf(hi[0], h.x); hi[1] = fmaxf(hi[1], h.y); hi[2] = fmaxf(hi[2], h.z); hi[3] = fmaxf(hi[3], h.w);
   }
   float st[4], zp[4];
 #pragma unroll
@@ -82,10 +91,11 @@ __device__ __forceinline__ void build_keys(const R2KBuild& b, int chunk, int hea
     st[e] = fmaxf(__fdiv_rn(__fsub_rn(hi[e], lo[e]), 15.f), 1.0e-6f);
     zp[e] = fminf(fmaxf(rintf(__fdiv_rn(-lo[e], st[e])), 0.f), 15.f);
   }
-  uint8_t* prow = b.k_packed + ((int64_t)head * b.k_capacity + (int64_t)chunk * kBuildRows + 32 * warp) * 64 + 2 * lane;
+  const int row = chunk * kBuildRows + kWarpRows * warp;
+  uint8_t* prow = b.k_packed + ((int64_t)head * b.k_capacity + row) * 64 + 2 * lane;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    if (src_row[32 * warp + i] < 0) continue;
+  for (int i = 0; i < kWarpRows; ++i) {
+    if (src_row[i] < 0) continue;
     float x[4];
     unpack4<BF16>(w[i], x);
     uint32_t out = 0;
@@ -93,8 +103,7 @@ __device__ __forceinline__ void build_keys(const R2KBuild& b, int chunk, int hea
     for (int e = 0; e < 4; ++e) out |= (uint32_t)fminf(fmaxf(rintf(__fadd_rn(__fdiv_rn(x[e], st[e]), zp[e])), 0.f), 15.f) << (4 * e);
     *reinterpret_cast<uint16_t*>(prow + i * 64) = (uint16_t)out;
   }
-  const int row = chunk * kBuildRows + 32 * warp;
-  if (row % b.k_block == 0 && src_row[32 * warp] >= 0) {
+  if (warp == first && src_row[0] >= 0) {
     const int64_t blk = (int64_t)head * (b.k_capacity / b.k_block) + row / b.k_block;
     *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(b.k_scale) + blk * 128 + 4 * lane) = make_uint2(pack_f16x2(st[0], st[1]), pack_f16x2(st[2], st[3]));
     *reinterpret_cast<uint32_t*>(b.k_zero + blk * 128 + 4 * lane) =
@@ -102,54 +111,66 @@ __device__ __forceinline__ void build_keys(const R2KBuild& b, int chunk, int hea
   }
 }
 
-// BF16: the values' type; CACHE_BF16: the cache's.
+// One value row: `row` counts in its pool.  BF16: the values' type; CACHE_BF16: the cache's.
 template <bool BF16, bool CACHE_BF16>
-__device__ __forceinline__ void build_values(const R2KBuild& b, int chunk, int head, const int* src_row) {
-  const int warp = (threadIdx.x >> 5) - 4, lane = threadIdx.x & 31;
-  const uint16_t* src = reinterpret_cast<const uint16_t*>(b.value) + (int64_t)head * b.rows * 128 + 4 * lane;
-  const int lanes = b.v2_group / 4;
-#pragma unroll 1
-  for (int i0 = 0; i0 < 32; i0 += 8) {
-    uint2 w[8];
+__device__ __forceinline__ void build_value_fp(const R2KBuild& b, int head, int row, uint2 v) {
+  const int lane = threadIdx.x & 31;
+  if (BF16 != CACHE_BF16) {
+    float x[4];
+    unpack4<BF16>(v, x);
+    v = CACHE_BF16 ? make_uint2(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3])) : make_uint2(pack_f16x2(x[0], x[1]), pack_f16x2(x[2], x[3]));
+  }
+  *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(b.fp_v) + ((int64_t)head * b.n_fp + row) * 128 + 4 * lane) = v;
+}
+template <bool BF16>
+__device__ __forceinline__ void build_value_int4(const R2KBuild& b, int head, int row, const uint2& v) {
+  const int lane = threadIdx.x & 31;
+  float sc;
+  const uint16_t out = encode_v_int4<BF16>(v, sc);
+  const int64_t at = (int64_t)head * b.n_i4 + row;
+  *reinterpret_cast<uint16_t*>(b.i4_packed + at * 64 + 2 * lane) = out;
+  if (lane == 0) b.i4_scale[at] = sc;
+}
+template <bool BF16>
+__device__ __forceinline__ void build_value_int2(const R2KBuild& b, int head, int row, const uint2& v) {
+  const int lane = threadIdx.x & 31, lanes = b.v2_group / 4;
+  float sc, zp;
+  const uint8_t out = encode_v_int2<BF16>(v, lanes, sc, zp);
+  const int64_t at = (int64_t)head * b.i2_capacity + row;
+  b.i2_packed[at * 32 + lane] = out;
+  if ((lane & (lanes - 1)) == 0) {
+    const int64_t m = at * (128 / b.v2_group) + lane / lanes;
+    reinterpret_cast<__half*>(b.i2_scale)[m] = __float2half_rn(sc);
+    b.i2_zero[m] = (uint8_t)zp;
+  }
+}
+
+// A warp whose rows are all of one pool (all but those at a pool's ends) works on them side by side: a row alone is a chain of
+// shuffles and divisions.
+template <bool BF16, bool CACHE_BF16>
+__device__ __forceinline__ void build_values(const R2KBuild& b, int chunk, int head, const int* src_row, const uint2 (&w)[kWarpRows]) {
+  const int row = chunk * kBuildRows + kWarpRows * (int)(threadIdx.x >> 5), i4 = row - b.n_fp, i2 = i4 - b.n_i4;
+  const bool whole = src_row[kWarpRows - 1] >= 0;   // rows behind the last token come last
+  if (whole && i4 + kWarpRows <= 0) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int s = src_row[32 * warp + i0 + k];
-      w[k] = s >= 0 ? __ldcs(reinterpret_cast<const uint2*>(src + (int64_t)s * 128)) : make_uint2(0u, 0u);
-    }
-#pragma unroll 1
-    for (int k = 0; k < 8; ++k) {
-      if (src_row[32 * warp + i0 + k] < 0) return;
-      uint2 v = w[0];
+    for (int i = 0; i < kWarpRows; ++i) build_value_fp<BF16, CACHE_BF16>(b, head, row + i, w[i]);
+  } else if (whole && i4 >= 0 && i2 + kWarpRows <= 0) {
 #pragma unroll
-      for (int j = 0; j < 7; ++j) w[j] = w[j + 1];   // the next row moves to the front: one copy of the code for eight rows
-      int row = chunk * kBuildRows + 32 * warp + i0 + k;
-      if (row < b.n_fp) {
-        if (BF16 != CACHE_BF16) {
-          float x[4];
-          unpack4<BF16>(v, x);
-          v = CACHE_BF16 ? make_uint2(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3])) : make_uint2(pack_f16x2(x[0], x[1]), pack_f16x2(x[2], x[3]));
-        }
-        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(b.fp_v) + ((int64_t)head * b.n_fp + row) * 128 + 4 * lane) = v;
-        continue;
-      }
-      row -= b.n_fp;
-      float sc, zp;
-      if (row < b.n_i4) {
-        const uint16_t out = encode_v_int4<BF16>(v, sc);
-        const int64_t at = (int64_t)head * b.n_i4 + row;
-        *reinterpret_cast<uint16_t*>(b.i4_packed + at * 64 + 2 * lane) = out;
-        if (lane == 0) b.i4_scale[at] = sc;
-        continue;
-      }
-      row -= b.n_i4;
-      const uint8_t out = encode_v_int2<BF16>(v, lanes, sc, zp);
-      const int64_t at = (int64_t)head * b.i2_capacity + row;
-      b.i2_packed[at * 32 + lane] = out;
-      if ((lane & (lanes - 1)) == 0) {
-        const int64_t m = at * (128 / b.v2_group) + lane / lanes;
-        reinterpret_cast<__half*>(b.i2_scale)[m] = __float2half_rn(sc);
-        b.i2_zero[m] = (uint8_t)zp;
-      }
+    for (int i = 0; i < kWarpRows; ++i) build_value_int4<BF16>(b, head, i4 + i, w[i]);
+  } else if (whole && i2 >= 0) {
+#pragma unroll
+    for (int i = 0; i < kWarpRows; ++i) build_value_int2<BF16>(b, head, i2 + i, w[i]);
+  } else {
+    uint2 v[kWarpRows];
+#pragma unroll
+    for (int i = 0; i < kWarpRows; ++i) v[i] = w[i];
+#pragma unroll 1
+    for (int i = 0; i < kWarpRows && src_row[i] >= 0; ++i) {
+      if (i4 + i < 0) build_value_fp<BF16, CACHE_BF16>(b, head, row + i, v[0]);
+      else if (i2 + i < 0) build_value_int4<BF16>(b, head, i4 + i, v[0]);
+      else build_value_int2<BF16>(b, head, i2 + i, v[0]);
+#pragma unroll
+      for (int j = 0; j < kWarpRows - 1; ++j) v[j] = v[j + 1];   // the next row moves to the front: one copy of the code
     }
   }
 }
@@ -157,7 +178,7 @@ __device__ __forceinline__ void build_values(const R2KBuild& b, int chunk, int h
 template <bool BF16, bool VALUES_BF16>
 __global__ void __launch_bounds__(kBuildThreads, 2) build_cache_kernel(const __grid_constant__ BuildArgs a) {
   __shared__ int src_row[kBuildRows];
-  __shared__ float range[4][128][2];
+  __shared__ float4 range[kBuildThreads / 32][2][32];
   const R2KBuild& b = a.b;
   int cta = blockIdx.x;
   if (cta == 0 && threadIdx.x == 0) *b.recent_len = 0;
@@ -173,8 +194,12 @@ __global__ void __launch_bounds__(kBuildThreads, 2) build_cache_kernel(const __g
       src_row[threadIdx.x] = s;
     }
     __syncthreads();
-    if (threadIdx.x < 128) build_keys<BF16>(b, chunk, head, src_row, range);
-    else build_values<VALUES_BF16, BF16>(b, chunk, head, src_row);
+    const int* mine = src_row + kWarpRows * (threadIdx.x >> 5);
+    uint2 k[kWarpRows], v[kWarpRows];
+    load_rows(b.key, b.rows, head, mine, k);
+    load_rows(b.value, b.rows, head, mine, v);   // on their way beside the keys' arithmetic
+    build_keys<BF16>(b, chunk, head, mine, k, range);
+    build_values<VALUES_BF16, BF16>(b, chunk, head, mine, v);
     return;
   }
   cta -= a.chunk_ctas;
