@@ -127,6 +127,15 @@ inline int64_t ceil_to(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // Tier of a page class: 0 bf16, 1 INT4, 2 INT2 values, 3 evicted (precision_pool.py:611-669; classes of PageClass).
 inline int tier_of(int64_t cls) { return cls == 1 || cls == 3 || cls == 4 ? 0 : cls == 2 ? 1 : cls == 5 ? 2 : 3; }
 
+// Bits in which p[0..n) differs from p[0], p[0] + 1, ...: zero for consecutive values.  Every token's two indices pass here on each
+// build: at one 64-bit word a step, two fifths of the host time of a 32768-token build.
+__attribute__((target_clones("avx512f", "avx2", "default"), optimize("O3"))) uint64_t off_ramp(const int64_t* p, int64_t n) {
+  const uint64_t first = (uint64_t)p[0];
+  uint64_t odd = 0;
+  for (int64_t k = 0; k < n; ++k) odd |= ((uint64_t)p[k] - first) ^ (uint64_t)k;
+  return odd;
+}
+
 // build_three_precision_cache behind its argument checks.  Returns (tensors in the order of `names` on the Python side,
 // n_fp, n_i4, n_i2).
 std::tuple<std::vector<at::Tensor>, int64_t, int64_t, int64_t> build_cache(
@@ -160,13 +169,8 @@ std::tuple<std::vector<at::Tensor>, int64_t, int64_t, int64_t> build_cache(
     global = host_i64(global);
     logical = host_i64(logical);
     const int64_t *g = global.data_ptr<int64_t>(), *l = logical.data_ptr<int64_t>();
-    for (int64_t i = 0; i < n && by_page; ++i) {
-      if (len[i] < 2) continue;
-      const int64_t *gp = g + off[i], *lp = l + off[i];
-      int64_t odd = 0;
-      for (int64_t k = 1; k < len[i]; ++k) odd |= (gp[k] - gp[0] - k) | (lp[k] - lp[0] - k);
-      by_page = odd == 0;
-    }
+    for (int64_t i = 0; i < n && by_page; ++i)
+      by_page = len[i] < 2 || (off_ramp(g + off[i], len[i]) | off_ramp(l + off[i], len[i])) == 0;
   }
   // the page table in pool order: R2KPage x (n + 1), then the two bases
   const int64_t words = (n + 1) + (by_page ? 2 * n : 0);
