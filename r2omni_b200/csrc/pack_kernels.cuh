@@ -456,8 +456,9 @@ template <bool BF16>
 __global__ void __launch_bounds__(128, 5) mrope_rows_kernel(MropeArgs a) {
   // The decode launch that follows on the stream may start its CTAs and prefetch pool tiles right away (it is
   // launched with programmatic stream serialization); it reads the rows written here only after its own
-  // dependency wait, i.e. after this grid has completed.
+  // dependency wait, i.e. after this grid has completed.  This kernel itself comes in behind a projection in the same way.
   launch_dependents();
+  grid_dependency_wait();
   const int s = threadIdx.x & 7;
   const int64_t n = (int64_t)a.batch * a.tokens;
   const int64_t first = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4;

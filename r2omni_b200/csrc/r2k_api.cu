@@ -319,10 +319,10 @@ int launch_mrope(MropeArgs& a, int32_t dtype, void* stream) {
   a.heads_per_warp = walks < 1 ? 1 : walks > heads ? heads : (int)walks;
   const dim3 grid((unsigned)((quads + 3) / 4), (unsigned)((heads + a.heads_per_warp - 1) / a.heads_per_warp));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == R2K_DTYPE_BF16) mrope_rows_kernel<true><<<grid, 128, 0, st>>>(a);
-  else mrope_rows_kernel<false><<<grid, 128, 0, st>>>(a);
+  const cudaError_t err = launch_behind(dtype == R2K_DTYPE_BF16 ? mrope_rows_kernel<true> : mrope_rows_kernel<false>, grid, dim3(128), st,
+                                        dev->pdl, a);
   ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
 }
 
 RingArgs ring_args(const R2KGeom* g, const R2KCacheView* v) {

@@ -45,3 +45,27 @@ def test_transforms_in_a_chain(rows):
     for _ in range(6):
         R.triton_fwht_128(got, output=got)   # in place: each reads what the one in front of it writes
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("tokens", [1, 37, 9000])
+def test_rotations_in_a_chain(tokens):
+    """Each rotation reads what the launch in front of it (a rotation, a transform, a matrix product) has just written."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    q, k = (torch.randn(2, h, tokens, 128, generator=g, device="cuda").to(torch.bfloat16) for h in (7, 2))
+    angle = torch.rand(3, 2, tokens, 128, generator=g, device="cuda")
+    cos, sin = angle.cos().to(torch.bfloat16), angle.sin().to(torch.bfloat16)
+    weight = torch.randn(128, 128, generator=g, device="cuda").to(torch.bfloat16) * 0.05
+
+    def steps(wait):
+        a, b = q, k
+        for _ in range(5):
+            for step in (lambda: R.qwen_qk_mrope(a, b, cos, sin, (16, 24, 24), apply_hadamard=True),
+                         lambda: (torch.nn.functional.linear(a, weight), R.triton_fwht_128(b)),
+                         lambda: R.qwen_qk_mrope(a, b, cos, sin, (16, 24, 24))):
+                a, b = step()
+                if wait:
+                    torch.cuda.synchronize()
+        return a, b
+
+    for want, got in zip(steps(True), steps(False)):
+        assert torch.equal(want, got)
