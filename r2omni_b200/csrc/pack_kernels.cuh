@@ -32,6 +32,7 @@ struct PackArgs {
   int64_t capacity;         // destination rows per head
   int64_t dst_start;
   int num_heads;
+  bool in_flush;            // the launch behind this one belongs to the same flush and may come in early
 };
 
 // ---- keys: per (head, block, channel) affine INT4 -------------------------
@@ -42,8 +43,9 @@ __global__ void __launch_bounds__(64) pack_k_int4_kernel(PackArgs a, uint8_t* pa
                                                          int64_t packed_bstride, int64_t scale_bstride, int64_t zero_bstride,
                                                          int k_block, int64_t first_block) {
   // A flush launches the value pack behind this kernel with programmatic stream serialization: the two read
-  // different halves of the residual window and write different arenas, so they may run side by side.
-  launch_dependents();
+  // different halves of the residual window and write different arenas, so they may run side by side.  By itself it lets nobody
+  // in: a rotation and the decode launch behind it may follow, and that one reads the pools before it waits.
+  if (a.in_flush) launch_dependents();
   const int64_t blk = first_block + blockIdx.x;
   const int head = blockIdx.y, req = blockIdx.z, c = threadIdx.x;
   const int64_t blocks_per_head = a.capacity / k_block;
@@ -178,7 +180,7 @@ template <bool BF16>
 __global__ void __launch_bounds__(128) pack_v_int2_kernel(PackArgs a, uint8_t* packed, __half* scale, uint8_t* zero,
                                                           int64_t packed_bstride, int64_t scale_bstride, int64_t zero_bstride,
                                                           int group) {
-  launch_dependents();   // in a flush the ring kernel follows; it waits for this grid before it touches the ring
+  if (a.in_flush) launch_dependents();   // the ring kernel follows; it waits for this grid before it touches the ring
   const int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (i < a.count) {
     const int head = blockIdx.y, req = blockIdx.z, lane = threadIdx.x & 31;

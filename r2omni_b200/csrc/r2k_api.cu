@@ -744,7 +744,7 @@ int r2k_pack_k_int4(const void* src, int32_t dtype, int32_t num_kv_heads, int64_
   if (!k_packed || !k_scale || !k_zero) return R2K_ERR_NULL;
   if (!pow2_in(k_block, 32, 64, 128) || k_capacity % k_block) return R2K_ERR_GEOMETRY;
   if (count == 0) return R2K_OK;
-  PackArgs a{reinterpret_cast<const uint16_t*>(src), 0, src_rows, index, count, k_capacity, dst_start, num_kv_heads};
+  PackArgs a{reinterpret_cast<const uint16_t*>(src), 0, src_rows, index, count, k_capacity, dst_start, num_kv_heads, false};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   return dtype == R2K_DTYPE_BF16 ? launch_pack_k<true>(a, 1, k_packed, k_scale, k_zero, 0, 0, 0, k_block, st)
                                  : launch_pack_k<false>(a, 1, k_packed, k_scale, k_zero, 0, 0, 0, k_block, st);
@@ -756,7 +756,7 @@ int r2k_pack_v_int4(const void* src, int32_t dtype, int32_t num_kv_heads, int64_
   if (rc) return rc;
   if (!packed || !scale) return R2K_ERR_NULL;
   if (count == 0) return R2K_OK;
-  PackArgs a{reinterpret_cast<const uint16_t*>(src), 0, src_rows, index, count, capacity, dst_start, num_kv_heads};
+  PackArgs a{reinterpret_cast<const uint16_t*>(src), 0, src_rows, index, count, capacity, dst_start, num_kv_heads, false};
   dim3 grid((unsigned)((count + 3) / 4), (unsigned)num_kv_heads, 1);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (dtype == R2K_DTYPE_BF16) pack_v_int4_kernel<true><<<grid, 128, 0, st>>>(a, packed, scale, 0, 0);
@@ -772,7 +772,7 @@ int r2k_pack_v_int2(const void* src, int32_t dtype, int32_t num_kv_heads, int64_
   if (!packed || !scale || !zero) return R2K_ERR_NULL;
   if (!pow2_in(group, 32, 64, 128)) return R2K_ERR_GEOMETRY;
   if (count == 0) return R2K_OK;
-  PackArgs a{reinterpret_cast<const uint16_t*>(src), 0, src_rows, index, count, capacity, dst_start, num_kv_heads};
+  PackArgs a{reinterpret_cast<const uint16_t*>(src), 0, src_rows, index, count, capacity, dst_start, num_kv_heads, false};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   return dtype == R2K_DTYPE_BF16 ? launch_pack_v2<true>(a, 1, packed, scale, zero, 0, 0, 0, group, st)
                                  : launch_pack_v2<false>(a, 1, packed, scale, zero, 0, 0, 0, group, st);
@@ -957,7 +957,7 @@ int r2k_flush_recent(const R2KGeom* geom, const R2KCacheView* view, int32_t ring
   if (rc) return rc;
   const bool bf16 = geom->dtype == R2K_DTYPE_BF16;
   PackArgs ka{reinterpret_cast<const uint16_t*>(view->recent_k), view->recent_k_bstride, geom->recent_capacity, nullptr,
-              flush_tokens, geom->k_capacity, k_dst, geom->num_kv_heads};
+              flush_tokens, geom->k_capacity, k_dst, geom->num_kv_heads, true};
   uint8_t* kp = const_cast<uint8_t*>(view->k_packed);
   void* ks = const_cast<void*>(view->k_scale);
   uint8_t* kz = const_cast<uint8_t*>(view->k_zero);
@@ -967,7 +967,7 @@ int r2k_flush_recent(const R2KGeom* geom, const R2KCacheView* view, int32_t ring
                                    geom->k_block, st);
   if (rc) return rc;
   PackArgs va{reinterpret_cast<const uint16_t*>(view->recent_v), view->recent_v_bstride, geom->recent_capacity, nullptr,
-              flush_tokens, geom->i2_capacity, v_dst, geom->num_kv_heads};
+              flush_tokens, geom->i2_capacity, v_dst, geom->num_kv_heads, true};
   uint8_t* vp = const_cast<uint8_t*>(view->i2_packed);
   void* vs = const_cast<void*>(view->i2_scale);
   uint8_t* vz = const_cast<uint8_t*>(view->i2_zero);
