@@ -363,7 +363,7 @@ __device__ __forceinline__ void qk_fp(uint32_t ka, const uint16_t* qrow, int t, 
   for (int i = 0; i < 4; ++i) {
     const uint4 ra = lds128(ka + 16 * i), rb = lds128(ka + 8 * 256 + 16 * i);
     uint4 qq = make_uint4(0u, 0u, 0u, 0u);
-    if (qrow != nullptr) qq = __ldg(reinterpret_cast<const uint4*>(qrow + 32 * t + 8 * i));
+    if (qrow != nullptr) qq = *reinterpret_cast<const uint4*>(qrow + 32 * t + 8 * i);
     if (BF16) {
       mma_bf16(acc, ra.x, rb.x, ra.y, rb.y, qq.x, qq.y);
       mma_bf16(acc, ra.z, rb.z, ra.w, rb.w, qq.z, qq.w);

@@ -340,10 +340,10 @@ __device__ __forceinline__ void commit_append(const DecodeParams& p, int b, int 
   if (has_append && warp == 5) {  // ring row rlen0 of head h
     const size_t src = ((size_t)b * p.g.num_kv_heads + h) * 256 + 8 * lane;
     const size_t dst = ((size_t)h * p.g.recent_capacity + rlen0) * 256 + 8 * lane;
-    *reinterpret_cast<uint2*>((uint8_t*)p.v.recent_k + (size_t)b * p.v.recent_k_bstride + dst) =
-        __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_k + src));
-    *reinterpret_cast<uint2*>((uint8_t*)p.v.recent_v + (size_t)b * p.v.recent_v_bstride + dst) =
-        __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_v + src));
+    const uint2 nk = *reinterpret_cast<const uint2*>((const uint8_t*)p.app_k + src);
+    const uint2 nv = *reinterpret_cast<const uint2*>((const uint8_t*)p.app_v + src);
+    *reinterpret_cast<uint2*>((uint8_t*)p.v.recent_k + (size_t)b * p.v.recent_k_bstride + dst) = nk;
+    *reinterpret_cast<uint2*>((uint8_t*)p.v.recent_v + (size_t)b * p.v.recent_v_bstride + dst) = nv;
   }
 }
 
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-      if (qrow != nullptr) raw = __ldg(reinterpret_cast<const uint4*>(qrow + 32 * t + 8 * i));
+      if (qrow != nullptr) raw = *reinterpret_cast<const uint4*>(qrow + 32 * t + 8 * i);
       const uint32_t wv[4] = {raw.x, raw.y, raw.z, raw.w};
       float f[8];
 #pragma unroll
@@ -787,10 +787,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
             const int app_row = rlen0 - win - r0;  // ring row that receives the appended token, relative to this slice
             if (has_append && app_row >= 0 && app_row < 16) {
               const size_t off = ((size_t)b * p.g.num_kv_heads + h) * 256 + 8 * lane;
-              *reinterpret_cast<uint2*>(sbp + kOffV + (r0 + app_row) * 256 + 8 * lane) =
-                  __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_k + off));
-              *reinterpret_cast<uint2*>(sbp + kOffV + kOffRecentV + (r0 + app_row) * 256 + 8 * lane) =
-                  __ldg(reinterpret_cast<const uint2*>((const uint8_t*)p.app_v + off));
+              const uint2 nk = *reinterpret_cast<const uint2*>((const uint8_t*)p.app_k + off);
+              const uint2 nv = *reinterpret_cast<const uint2*>((const uint8_t*)p.app_v + off);
+              *reinterpret_cast<uint2*>(sbp + kOffV + (r0 + app_row) * 256 + 8 * lane) = nk;
+              *reinterpret_cast<uint2*>(sbp + kOffV + kOffRecentV + (r0 + app_row) * 256 + 8 * lane) = nv;
             }
             for (int i = hi; CLUSTER && i < 16; ++i)   // rows behind the window's last one: 0 * NaN must not reach a value
               *reinterpret_cast<uint2*>(sbp + kOffV + kOffRecentV + (r0 + i) * 256 + 8 * lane) = make_uint2(0u, 0u);
@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
 // ---------------------------------------------------------------------------
 // cross-shard merge of un-normalised states
 // ---------------------------------------------------------------------------
-__global__ void merge_states_kernel(const float* __restrict__ states, int num_states, int64_t state_stride, int rows,
+__global__ void merge_states_kernel(const float* states, int num_states, int64_t state_stride, int rows,
                                     int dtype, void* out, uint32_t flags) {
   // Launched with programmatic stream serialization: only the way here overlaps the decode launch in front (25.3 -> 23.7 us for a shard
   // of 131072 tokens).  It lets nobody in early: with the next decode launch fetching beside the tail of a long one, a shard of 1 M

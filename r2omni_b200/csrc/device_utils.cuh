@@ -213,7 +213,15 @@ __device__ __forceinline__ void st_cluster_f4(uint32_t a, float4 v) {
 // Programmatic dependent launch.  launch_dependents lets the next kernel of the stream (when it was launched with
 // programmatic stream serialization) start its CTAs on SMs this grid has left; grid_dependency_wait blocks until
 // every kernel this grid depends on has completed and its writes are visible.  Both are no-ops otherwise.
+// A grid that came in early reads what the kernel in front writes behind the wait and with ordinary loads: the read-only path
+// (__ldg, const __restrict__) is for memory that nobody writes while the grid runs, and no barrier orders it.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// 16 bytes that are read once; stays behind the wait (both are volatile).
+__device__ __forceinline__ uint4 ld_streamed(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 
 }  // namespace r2k

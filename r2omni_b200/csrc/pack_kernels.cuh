@@ -331,7 +331,7 @@ __device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
 }
 // 16 bytes at a pointer that is a multiple of 16 (wide) or of 8 bytes
 __device__ __forceinline__ uint4 load16(const uint16_t* p, bool wide) {
-  if (wide) return __ldcs(reinterpret_cast<const uint4*>(p));   // every row is touched once
+  if (wide) return ld_streamed(p);   // every row is touched once
   const uint2 a = *reinterpret_cast<const uint2*>(p), b = *reinterpret_cast<const uint2*>(p + 4);
   return make_uint4(a.x, a.y, b.x, b.y);
 }
@@ -436,11 +436,11 @@ __device__ __forceinline__ void load_table8(const MropeArgs& a, const void* base
     const int axis = sd < a.section0 ? 0 : (sd < a.section0 + a.section1 ? 1 : 2);
     const int64_t i = at + axis * stride[0] + d0;
     if (a.rot_dtype == 2) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i));
-      const float4 w = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i) + 1);
+      const float4* row = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i);
+      const float4 u = row[0], w = row[1];
       x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
     } else {
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + i));
+      const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + i);
       if (a.rot_dtype == R2K_DTYPE_BF16) unpack8<true>(u, x); else unpack8<false>(u, x);
     }
     return;
