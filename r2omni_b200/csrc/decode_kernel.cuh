@@ -172,6 +172,9 @@ __device__ __forceinline__ void produce_tile(const DecodeParams& p, const Tile& 
   }
   __syncwarp();
   if (lane == 0) mbar_arrive_expect_tx(bar, tx);
+  // plain stores above, bulk copies of a later tile into the same stage: issued by lane 0, so every lane passes here first
+  fence_async_shared();
+  __syncwarp();
 }
 
 // Per-(request, kv head) source bases, biased so that a key-arena row index addresses every array of its pool.
@@ -785,7 +788,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
           const int hi = min(rlen - win - r0, 16);
           if (hi > 0) {
             const int app_row = rlen0 - win - r0;  // ring row that receives the appended token, relative to this slice
-            if (has_append && app_row >= 0 && app_row < 16) {
+            const bool takes_row = has_append && app_row >= 0 && app_row < 16;
+            if (takes_row) {
               const size_t off = ((size_t)b * p.g.num_kv_heads + h) * 256 + 8 * lane;
               const uint2 nk = *reinterpret_cast<const uint2*>((const uint8_t*)p.app_k + off);
               const uint2 nv = *reinterpret_cast<const uint2*>((const uint8_t*)p.app_v + off);
@@ -794,6 +798,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
             }
             for (int i = hi; CLUSTER && i < 16; ++i)   // rows behind the window's last one: 0 * NaN must not reach a value
               *reinterpret_cast<uint2*>(sbp + kOffV + kOffRecentV + (r0 + i) * 256 + 8 * lane) = make_uint2(0u, 0u);
+            // the plain stores above, before the producer's next copies into the stage (this head's or the next one's)
+            if (takes_row || (CLUSTER && hi < 16)) fence_async_shared();
             __syncwarp();
             const int t0 = 2 * t + (t & 1), t1 = 2 * t + 1 - (t & 1);
             float s[1][4];
@@ -804,7 +810,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
                                s[0]);
           }
         }
-        if (CLUSTER) fence_async_shared();   // the plain stores above, before the producer's next copies into the stage
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty_bar[stage]);
       }
