@@ -321,8 +321,8 @@ __device__ __forceinline__ void store_row(float* slot, int hh, int sub, float mx
   if (sub == 0) __stcg(reinterpret_cast<float2*>(orow), make_float2(mx, lsum));
 }
 
-// Every CTA of (b, h) has read recent_len[b]: its consumers, and its producer before a tile that they wait for (a cluster's
-// producer does not read it).  The loads have returned, so no fence is wanted in front of the count.  One thread outside the
+// Every CTA of (b, h) has read recent_len[b]: its consumers, and its producer, where it does, before a tile that they
+// wait for.  The loads have returned, so no fence is wanted in front of the count.  One thread outside the
 // merge workers counts the head in; the last head of the request moves the ring metadata; another warp writes the new rows.
 static_assert(kNW >= 6, "warps 4 and 5 carry the request counter and the appended rows");
 __device__ __forceinline__ void commit_append(const DecodeParams& p, int b, int h, int rlen0) {
@@ -623,8 +623,8 @@ __device__ __forceinline__ void consume_pool(WarpState& st, const DecodeParams& 
 // kernel
 // ---------------------------------------------------------------------------
 // CLUSTER: launched in clusters of kCluster CTAs, one (request, kv head) each (a template parameter: the branch alone
-// cost the other launches 1 %).
-template <bool BF16, bool CLUSTER>
+// cost the other launches 1 %).  WHOLE_WINDOW: see window_comes_whole (a branch on it cost the short launches 2 %).
+template <bool BF16, bool CLUSTER, bool WHOLE_WINDOW>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __grid_constant__ DecodeParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* stages = smem;
@@ -673,10 +673,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
       const TileSources src = tile_sources(p, b, h);
       for (int u = u0; u < u1; ++u) {
         const Tile tl = tile_of(p, u);
-        if (CLUSTER && tl.pool == 3) {
-          // The window belongs to the previous step until that has completed.  Its tiles come whole, whatever its length: a load of
-          // the length in front of them is another trip to memory on the way of a short launch.
-          grid_dependency_wait();
+        if (WHOLE_WINDOW && tl.pool == 3) {
+          grid_dependency_wait();   // the window belongs to the previous step until that has completed
         } else if (tl.pool == 3) {
           // Tiles without rows are left out, except the first one of a CTA's range (it brings rows that nobody counts):
           // producer and consumers each read recent_len, the last head of the request to finish raises it, and only a tile
@@ -689,7 +687,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
             rlen = *reinterpret_cast<const int*>((const uint8_t*)p.v.recent_len + (size_t)b * p.v.recent_len_bstride) +
                    (has_append ? 1 : 0);
           }
-          if (tl.win >= rlen && !first) continue;
+          if (!window_tile_comes(false, tl.win, rlen, first)) continue;
         }
         if (!mbar_wait_relaxed(&empty_bar[stage], phase ^ 1u)) {
           if (lane == 0) atomicExch(p.err, R2K_ERR_DEVICE_TIMEOUT);
@@ -775,7 +773,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
     for (int u = first_residual; u < u1; ++u) {
       const int ur = u - p.nF - p.n4 - p.n2;
       const int win = ur * kTR;
-      if (!CLUSTER && win >= rlen && u != first_residual) continue;   // as the producer does
+      if (!window_tile_comes(WHOLE_WINDOW, win, rlen, u == first_residual)) continue;   // as the producer does
       if (alive && !mbar_wait(&full_bar[stage], phase)) {
         if (lane == 0) atomicExch(p.err, R2K_ERR_DEVICE_TIMEOUT);
         alive = false;

@@ -40,8 +40,9 @@ int device_info(DeviceInfo** out) {
       cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       return true;
     };
-    if (!prepare(decode_kernel<true, false>, kSmemBytes) || !prepare(decode_kernel<false, false>, kSmemBytes) ||
-        !prepare(decode_kernel<true, true>, kClusterSmemBytes) || !prepare(decode_kernel<false, true>, kClusterSmemBytes))
+    if (!prepare(decode_kernel<true, false, false>, kSmemBytes) || !prepare(decode_kernel<false, false, false>, kSmemBytes) ||
+        !prepare(decode_kernel<true, true, true>, kClusterSmemBytes) || !prepare(decode_kernel<false, true, true>, kClusterSmemBytes) ||
+        !prepare(decode_kernel<true, true, false>, kClusterSmemBytes) || !prepare(decode_kernel<false, true, false>, kClusterSmemBytes))
       return R2K_ERR_CUDA;
     d.sms = sms;
     cudaLaunchAttribute attr[1];
@@ -53,7 +54,7 @@ int device_info(DeviceInfo** out) {
     cfg.dynamicSmemBytes = kClusterSmemBytes;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&d.clusters, decode_kernel<true, true>, &cfg) != cudaSuccess) { cudaGetLastError(); d.clusters = 0; }
+    if (cudaOccupancyMaxActiveClusters(&d.clusters, decode_kernel<true, true, true>, &cfg) != cudaSuccess) { cudaGetLastError(); d.clusters = 0; }
     const char* off = std::getenv("R2K_DISABLE_PDL");
     d.pdl = !(off != nullptr && off[0] == '1');
     d.ready = true;
@@ -511,8 +512,9 @@ static int decode_impl(const R2KGeom* geom, const R2KCacheView* view, const void
     cfg.dynamicSmemBytes = kClusterSmemBytes;
   }
   const bool bf16 = geom->dtype == R2K_DTYPE_BF16;
-  const auto kernel = p.cluster ? (bf16 ? decode_kernel<true, true> : decode_kernel<false, true>)
-                                : (bf16 ? decode_kernel<true, false> : decode_kernel<false, false>);
+  const auto kernel = window_comes_whole(p, p.cluster != 0) ? (bf16 ? decode_kernel<true, true, true> : decode_kernel<false, true, true>)
+                      : p.cluster                           ? (bf16 ? decode_kernel<true, true, false> : decode_kernel<false, true, false>)
+                                                            : (bf16 ? decode_kernel<true, false, false> : decode_kernel<false, false, false>);
   const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, p);
   ++g_launches;
   return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;

@@ -3,7 +3,8 @@ not reach the result, whatever they hold."""
 import pytest
 import torch
 
-from gpu_helpers import make_executor
+from gpu_helpers import assert_close, build_gpu_cache, make_executor
+from oracle import sspa_oracle as O
 from test_gpu_decode import both_caches, seeded_classes
 
 pytestmark = pytest.mark.gpu
@@ -39,4 +40,32 @@ def test_rows_behind_the_window_do_not_count(length, dtype):
             assert int(a.recent_len_device) == length + 1
             assert torch.equal(a.recent_k[:, :, length], rows_k[:, :, length]) and torch.equal(a.recent_v[:, :, length], rows_v[:, :, length])
         assert torch.isfinite(outs[0].float()).all() and torch.equal(outs[0], outs[1])
+    assert ex.device_status() == 0
+
+
+@pytest.mark.parametrize("ring", [192, 1024])   # three tiles, and more than a cluster has CTAs
+@pytest.mark.parametrize("length", [0, 1, 63, 64, 65, 128, 150, 191])
+def test_long_windows_of_small_caches(length, ring):
+    """Windows of more than two tiles come without the tiles behind their length; the appended row may open a tile."""
+    pages, heads = 9, 3
+    g = torch.Generator().manual_seed(ring + length)
+    key, value = (torch.randn(heads, pages * 32, 128, generator=g).to(torch.bfloat16) for _ in range(2))
+    rows_k, rows_v = (torch.randn(1, heads, length + 1, 128, generator=g).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(1, 5 * heads, 128, generator=g).to(torch.bfloat16)
+    classes = seeded_classes(pages, 3)
+    ocache = O.build_cache(key, value, classes, page_size=32, recent_capacity=ring, append_capacity=256)
+    cache = build_gpu_cache(key, value, classes, page_size=32, recent_capacity=ring, append_capacity=256)
+    a, ex = cache.arenas, make_executor(cache, 5 * heads)
+    for t, rows in ((a.recent_k, rows_k), (a.recent_v, rows_v)):
+        t.fill_(float("nan"))
+        t[:, :, :length] = rows[:, :, :length].cuda()
+    for i in range(length):
+        O.append_token(ocache, rows_k[0, :, i], rows_v[0, :, i], 500 + i, 500 + i)
+    a.recent_len_device.fill_(length)
+    a.recent_len = length
+    assert_close(ex.decode_f32(q.cuda()), O.decode_fp32(q.float(), ocache), "window")
+    O.append_token(ocache, rows_k[0, :, length], rows_v[0, :, length], 900, 900)
+    step = tuple(t[:, :, length].cuda().contiguous() for t in (rows_k, rows_v))
+    assert_close(ex.decode_f32(q.cuda(), append=(*step, 900, 900)), O.decode_fp32(q.float(), ocache), "appended")
+    assert int(a.recent_len_device) == length + 1 and torch.equal(a.recent_k[:, :, length], step[0]) and torch.equal(a.recent_v[:, :, length], step[1])
     assert ex.device_status() == 0
