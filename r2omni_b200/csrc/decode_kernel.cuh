@@ -794,10 +794,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
               *reinterpret_cast<uint2*>(sbp + kOffV + (r0 + app_row) * 256 + 8 * lane) = nk;
               *reinterpret_cast<uint2*>(sbp + kOffV + kOffRecentV + (r0 + app_row) * 256 + 8 * lane) = nv;
             }
-            for (int i = hi; CLUSTER && i < 16; ++i)   // rows behind the window's last one: 0 * NaN must not reach a value
+            for (int i = hi; i < 16; ++i)   // rows behind the window's last one: 0 * NaN must not reach a value
               *reinterpret_cast<uint2*>(sbp + kOffV + kOffRecentV + (r0 + i) * 256 + 8 * lane) = make_uint2(0u, 0u);
             // the plain stores above, before the producer's next copies into the stage (this head's or the next one's)
-            if (takes_row || (CLUSTER && hi < 16)) fence_async_shared();
+            if (takes_row || hi < 16) fence_async_shared();
             __syncwarp();
             const int t0 = 2 * t + (t & 1), t1 = 2 * t + 1 - (t & 1);
             float s[1][4];

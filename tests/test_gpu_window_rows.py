@@ -69,3 +69,29 @@ def test_long_windows_of_small_caches(length, ring):
     assert_close(ex.decode_f32(q.cuda(), append=(*step, 900, 900)), O.decode_fp32(q.float(), ocache), "appended")
     assert int(a.recent_len_device) == length + 1 and torch.equal(a.recent_k[:, :, length], step[0]) and torch.equal(a.recent_v[:, :, length], step[1])
     assert ex.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,cap", [(3, 3), (3, 20), (24, None)])   # a CTA per head, several, a grid of more heads than clusters
+@pytest.mark.parametrize("length", [0, 1, 15, 16, 17, 63, 64, 65, 127])
+def test_rows_behind_the_window_of_the_general_launch(length, heads, cap, dtype, monkeypatch):
+    """A window's tile comes whole in every launch, and the memory behind its last row is the caller's."""
+    pages = 9
+    _, cache, new_k, new_v, queries = both_caches(7, hq=5 * heads, hkv=heads, tokens=pages * 32, page=32,
+                                                  classes=seeded_classes(pages, 3), appends=length + 1, dtype=dtype, append_capacity=256)
+    if cap:
+        monkeypatch.setenv("R2K_GRID_CAP", str(cap))
+    ex, a, q = make_executor(cache, 5 * heads), cache.arenas, queries[0].cuda()
+    rows = [t.transpose(0, 1).unsqueeze(0)[:, :, :length].cuda() for t in (new_k, new_v)]
+    step = (new_k[length].unsqueeze(0).cuda().contiguous(), new_v[length].unsqueeze(0).cuda().contiguous(), 500, 500)
+    for append in (None, step):
+        outs = []
+        for rest in (0.0, float("inf"), float("nan")):
+            for t, r in zip((a.recent_k, a.recent_v), rows):
+                t.fill_(rest)
+                t[:, :, :length] = r
+            a.recent_len_device.fill_(length)
+            a.recent_len = length
+            outs.append(ex.decode_f32(q, append=append).clone())
+        assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    assert ex.device_status() == 0
