@@ -322,13 +322,14 @@ __device__ __forceinline__ void store_row(float* slot, int hh, int sub, float mx
 }
 
 // Every CTA of (b, h) has read recent_len[b]: its consumers, and its producer, where it does, before a tile that they
-// wait for.  The loads have returned, so no fence is wanted in front of the count.  One thread outside the
+// wait for.  The ticket (in a cluster, its barrier) orders those reads before this call, and each head's count releases and
+// acquires, so that all heads' reads come before the store of the raised length.  One thread outside the
 // merge workers counts the head in; the last head of the request moves the ring metadata; another warp writes the new rows.
 static_assert(kNW >= 6, "warps 4 and 5 carry the request counter and the appended rows");
 __device__ __forceinline__ void commit_append(const DecodeParams& p, int b, int h, int rlen0) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool has_append = p.app_k != nullptr;
-  if (threadIdx.x == 128 && atomicAdd(&p.req_counter[b], 1) == p.g.num_kv_heads - 1) {
+  if (threadIdx.x == 128 && atomic_add_acq_rel(&p.req_counter[b], 1) == p.g.num_kv_heads - 1) {
     p.req_counter[b] = 0;
     if (has_append) {
       const int64_t gi = p.app_idx ? p.app_idx[2 * b] : p.app_global;
@@ -875,17 +876,15 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) decode_kernel(const __gr
     }
     if (CLUSTER) {
       // ---- one exact merge through distributed shared memory: the CTA of rank r merges head r of the group ----
-      // A round of remote stores and one cluster barrier where the path below pays a store, a fence, a ticket and a round of loads
-      // through L2, and nobody's shared memory is touched by others behind that barrier.  The append goes ahead beside the merge.
-      // (Partials read out of the other CTAs, a barrier in front of the exit, the append behind the merge and the length read in front
-      // of the window's copies: 239.9 us for 36 launches of 701 tokens x 2 heads, 316.9 of 4096; so 224.5 and 309.7.)  A cluster's
-      // CTAs hold one (request, kv head) each, so all of them come here once.
+      // A round of remote stores between two cluster barriers (the first, arrived at before the fold above, says that every inbox
+      // is there and the length read) where the path below pays a store, a fence, a ticket and a round of loads
+      // through L2, and nobody's shared memory is touched by others behind them.  The append goes ahead beside the merge, behind its
+      // warps' arrival: 36 launches of 701 tokens x 2 heads take 218 us, 239 with its count in front of the arrival (4096 tokens: 305
+      // and 323).  A cluster's CTAs hold one (request, kv head) each, so all of them come here once.
       const int rank = (int)cluster_rank();
-      if (!worker) {
-        cluster_wait();
-        if (rank == 0) commit_append(p, b, h, rlen0);
-      }
+      if (!worker) cluster_wait();
       cluster_arrive();
+      if (!worker && rank == 0) commit_append(p, b, h, rlen0);
       cluster_wait();
       if (warp == 0) {   // both halves of the warp do the same; the lower one stores
         const int sub = lane & 15;

@@ -187,6 +187,14 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Counts in with what this thread has seen and done (a CTA's other threads' reads and writes in front of a barrier included) and
+// takes over what those that counted in before have.
+__device__ __forceinline__ int atomic_add_acq_rel(int* p, int x) {
+  int old;
+  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;\n" : "=r"(old) : "l"(p), "r"(x) : "memory");
+  return old;
+}
+
 // Thread-block clusters.  An arrival releases, a wait acquires: what any thread of the cluster wrote to its shared memory
 // before it arrived can be read by all of them behind the wait.  Threads that have exited do not count.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
