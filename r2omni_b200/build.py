@@ -52,7 +52,7 @@ def _build_host(force: bool) -> None:
     includes = (os.path.join(ROOT, "include"), os.path.join(torch_dir, "include"),
                 os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), os.path.join(cuda_home, "include"),
                 sysconfig.get_paths()["include"])
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=_r2k_host",
+    cmd = ["g++", "-O3", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=_r2k_host",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
     for path in includes:
         cmd += ["-isystem" if "torch" in path else "-I", path]
