@@ -16,6 +16,17 @@ namespace {
 
 std::atomic<uint64_t> g_launches{0};
 
+// A failed call's error is taken out of the runtime here: left there, the next launch's cudaGetLastError() would report it.
+bool ok(cudaError_t err) {
+  if (err == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+int launched(cudaError_t err) {
+  ++g_launches;
+  return ok(err) ? R2K_OK : R2K_ERR_CUDA;
+}
+
 struct DeviceInfo {
   int sms = 0;
   int clusters = 0;   // decode clusters that fit on the device at once
@@ -29,15 +40,15 @@ std::mutex g_dev_mutex;
 // two host threads may race here.
 int device_info(DeviceInfo** out) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return R2K_ERR_CUDA;
+  if (!ok(cudaGetDevice(&dev)) || dev < 0 || dev >= 64) return R2K_ERR_CUDA;
   DeviceInfo& d = g_dev[dev];
   std::lock_guard<std::mutex> lock(g_dev_mutex);
   if (!d.ready) {
     int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return R2K_ERR_CUDA;
+    if (!ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) || sms <= 0) return R2K_ERR_CUDA;
     auto prepare = [](auto kernel, int smem) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
-      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      if (!ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) return false;
+      ok(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));   // a preference
       return true;
     };
     if (!prepare(decode_kernel<true, false, false>, kSmemBytes) || !prepare(decode_kernel<false, false, false>, kSmemBytes) ||
@@ -54,7 +65,7 @@ int device_info(DeviceInfo** out) {
     cfg.dynamicSmemBytes = kClusterSmemBytes;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&d.clusters, decode_kernel<true, true, true>, &cfg) != cudaSuccess) { cudaGetLastError(); d.clusters = 0; }
+    if (!ok(cudaOccupancyMaxActiveClusters(&d.clusters, decode_kernel<true, true, true>, &cfg))) d.clusters = 0;
     const char* off = std::getenv("R2K_DISABLE_PDL");
     d.pdl = !(off != nullptr && off[0] == '1');
     d.ready = true;
@@ -224,7 +235,7 @@ EncodeTiledFn encode_tiled_fn() {
   static EncodeTiledFn fn = [] {
     void* sym = nullptr;
     cudaDriverEntryPointQueryResult res;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &res) != cudaSuccess ||
+    if (!ok(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &res)) ||
         res != cudaDriverEntryPointSuccess)
       sym = nullptr;
     return reinterpret_cast<EncodeTiledFn>(sym);
@@ -268,8 +279,7 @@ int launch_pack_k(const PackArgs& a, int batch, uint8_t* packed, void* scale, ui
   const int64_t first = a.dst_start / k_block, last = (a.dst_start + a.count - 1) / k_block;
   dim3 grid((unsigned)(last - first + 1), (unsigned)a.num_heads, (unsigned)batch);
   pack_k_int4_kernel<BF16><<<grid, 64, (size_t)k_block * 256, st>>>(a, packed, reinterpret_cast<__half*>(scale), zero, pb, sb, zb, k_block, first);
-  ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(cudaGetLastError());
 }
 // A launch that may start while the kernel in front of it on the stream is still running, once that kernel has
 // let its dependents go (programmatic stream serialization); `overlap` false gives an ordinary launch.
@@ -293,8 +303,7 @@ int launch_pack_v2(const PackArgs& a, int batch, uint8_t* packed, void* scale, u
   dim3 grid((unsigned)((a.count + 3) / 4), (unsigned)a.num_heads, (unsigned)batch);
   const cudaError_t err = launch_behind(pack_v_int2_kernel<BF16>, grid, dim3(128), st, overlap, a, packed,
                                         reinterpret_cast<__half*>(scale), zero, pb, sb, zb, group);
-  ++g_launches;
-  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(err);
 }
 
 // Whether eight channels of a table row are whole aligned 16-byte words of one axis (see load_table8).
@@ -322,8 +331,7 @@ int launch_mrope(MropeArgs& a, int32_t dtype, void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const cudaError_t err = launch_behind(dtype == R2K_DTYPE_BF16 ? mrope_rows_kernel<true> : mrope_rows_kernel<false>, grid, dim3(128), st,
                                         dev->pdl, a);
-  ++g_launches;
-  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(err);
 }
 
 RingArgs ring_args(const R2KGeom* g, const R2KCacheView* v) {
@@ -411,7 +419,7 @@ int r2k_decode_workspace_init(void* workspace, size_t bytes, void* stream) {
   if (bytes < (size_t)kWsHeaderBytes) return R2K_ERR_WORKSPACE;
   // header + counters: clear everything in front of the partial slots that this workspace could ever hold
   size_t n = bytes < (size_t)(1 << 20) ? bytes : (size_t)(1 << 20);
-  return cudaMemsetAsync(workspace, 0, n, reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return ok(cudaMemsetAsync(workspace, 0, n, reinterpret_cast<cudaStream_t>(stream))) ? R2K_OK : R2K_ERR_CUDA;
 }
 
 static size_t exchange_states_bytes(const R2KGeom* g, int world) {
@@ -516,8 +524,7 @@ static int decode_impl(const R2KGeom* geom, const R2KCacheView* view, const void
                       : p.cluster                           ? (bf16 ? decode_kernel<true, true, false> : decode_kernel<false, true, false>)
                                                             : (bf16 ? decode_kernel<true, false, false> : decode_kernel<false, false, false>);
   const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, p);
-  ++g_launches;
-  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(err);
 }
 
 int r2k_decode(const R2KGeom* geom, const R2KCacheView* view, const void* q, const R2KAppend* append, void* workspace,
@@ -569,7 +576,7 @@ int r2k_decode_host(const R2KGeom* geom, const R2KCacheView* view, const void* h
   static const int zero_copy = [] { const char* e = getenv("R2K_HOST_ZERO_COPY"); return e ? atoi(e) : kHostZeroCopyDefault; }();
   auto mapped = [](const void* p) -> uint8_t* {
     cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (!ok(cudaPointerGetAttributes(&a, p))) return nullptr;
     return a.type == cudaMemoryTypeHost ? static_cast<uint8_t*>(a.devicePointer) : nullptr;
   };
   uint8_t* in = (zero_copy & 1) ? mapped(host_in) : nullptr;
@@ -582,9 +589,8 @@ int r2k_decode_host(const R2KGeom* geom, const R2KCacheView* view, const void* h
     if (src != nullptr && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {   // bit 2: a copy kernel the decode launch overlaps
       const int n16 = (int)(in_bytes / 16);
       host_block_copy_kernel<<<(n16 + 255) / 256, 256, 0, st>>>(reinterpret_cast<const uint4*>(src), reinterpret_cast<uint4*>(dev), n16);
-      ++g_launches;
-      if (cudaGetLastError() != cudaSuccess) return R2K_ERR_CUDA;
-    } else if (cudaMemcpyAsync(dev, host_in, in_bytes, cudaMemcpyHostToDevice, st) != cudaSuccess) {
+      if (launched(cudaGetLastError()) != R2K_OK) return R2K_ERR_CUDA;
+    } else if (!ok(cudaMemcpyAsync(dev, host_in, in_bytes, cudaMemcpyHostToDevice, st))) {
       return R2K_ERR_CUDA;
     }
     in = dev;
@@ -598,9 +604,9 @@ int r2k_decode_host(const R2KGeom* geom, const R2KCacheView* view, const void* h
   const int status = decode_impl(geom, view, in, append ? &dev_append : nullptr, workspace, workspace_bytes,
                                  out ? out : dev + s.out_off, flags, nullptr, stream);
   if (status != R2K_OK) return status;
-  if (out == nullptr && cudaMemcpyAsync(host_out, dev + s.out_off, out_bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+  if (out == nullptr && !ok(cudaMemcpyAsync(host_out, dev + s.out_off, out_bytes, cudaMemcpyDeviceToHost, st)))
     return R2K_ERR_CUDA;
-  return cudaStreamSynchronize(st) == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return ok(cudaStreamSynchronize(st)) ? R2K_OK : R2K_ERR_CUDA;
 }
 
 int r2k_decode_exchange(const R2KGeom* geom, const R2KCacheView* view, const void* q, const R2KAppend* append, void* workspace,
@@ -624,9 +630,9 @@ int r2k_exchange_create(size_t bytes, void** buffer, unsigned char handle[64]) {
   static_assert(sizeof(cudaIpcMemHandle_t) == 64, "inter-process handle size");
   if (bytes == 0) return R2K_ERR_GEOMETRY;
   void* ptr = nullptr;
-  if (cudaMalloc(&ptr, bytes) != cudaSuccess) return R2K_ERR_CUDA;
+  if (!ok(cudaMalloc(&ptr, bytes))) return R2K_ERR_CUDA;
   cudaIpcMemHandle_t h;
-  if (cudaMemset(ptr, 0, bytes) != cudaSuccess || cudaIpcGetMemHandle(&h, ptr) != cudaSuccess) {
+  if (!ok(cudaMemset(ptr, 0, bytes)) || !ok(cudaIpcGetMemHandle(&h, ptr))) {
     cudaFree(ptr);
     return R2K_ERR_CUDA;
   }
@@ -640,7 +646,7 @@ int r2k_exchange_open(const unsigned char handle[64], void** buffer) {
   cudaIpcMemHandle_t h;
   std::memcpy(&h, handle, 64);
   void* ptr = nullptr;
-  if (cudaIpcOpenMemHandle(&ptr, h, cudaIpcMemLazyEnablePeerAccess) != cudaSuccess) return R2K_ERR_CUDA;
+  if (!ok(cudaIpcOpenMemHandle(&ptr, h, cudaIpcMemLazyEnablePeerAccess))) return R2K_ERR_CUDA;
   *buffer = ptr;
   return R2K_OK;
 }
@@ -648,7 +654,7 @@ int r2k_exchange_open(const unsigned char handle[64], void** buffer) {
 int r2k_exchange_close(void* buffer, int32_t opened) {
   if (buffer == nullptr) return R2K_OK;
   const cudaError_t e = opened ? cudaIpcCloseMemHandle(buffer) : cudaFree(buffer);
-  return e == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return ok(e) ? R2K_OK : R2K_ERR_CUDA;
 }
 
 }  // extern "C"
@@ -666,12 +672,12 @@ constexpr size_t kStaticHeadBytes = kWsHeaderBytes + kWsCounterBlockBytes;   // 
 // (cudaGetSymbolAddress with that device current) and clears the status word and the counters on `stream`.
 int static_workspace(void** out, cudaStream_t stream) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return R2K_ERR_CUDA;
+  if (!ok(cudaGetDevice(&dev)) || dev < 0 || dev >= 64) return R2K_ERR_CUDA;
   std::lock_guard<std::mutex> lock(g_static_mutex);
   if (g_static_ptr[dev] == nullptr) {
     void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_static_workspace) != cudaSuccess || p == nullptr) return R2K_ERR_CUDA;
-    if (cudaMemsetAsync(p, 0, kStaticHeadBytes, stream) != cudaSuccess) return R2K_ERR_CUDA;
+    if (!ok(cudaGetSymbolAddress(&p, g_static_workspace)) || p == nullptr) return R2K_ERR_CUDA;
+    if (!ok(cudaMemsetAsync(p, 0, kStaticHeadBytes, stream))) return R2K_ERR_CUDA;
     g_static_ptr[dev] = p;
   }
   *out = g_static_ptr[dev];
@@ -704,14 +710,14 @@ int r2k_decode_static_reset(void* stream) {
   void* ptr = nullptr;
   const int rc = static_workspace(&ptr, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
-  return cudaMemsetAsync(ptr, 0, kStaticHeadBytes, reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return ok(cudaMemsetAsync(ptr, 0, kStaticHeadBytes, reinterpret_cast<cudaStream_t>(stream))) ? R2K_OK : R2K_ERR_CUDA;
 }
 
 int r2k_decode_device_status(void* workspace, int32_t* status, void* stream) {
   if (workspace == nullptr || status == nullptr) return R2K_ERR_NULL;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (cudaMemcpyAsync(status, workspace, sizeof(int32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess) return R2K_ERR_CUDA;
-  return cudaStreamSynchronize(st) == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  if (!ok(cudaMemcpyAsync(status, workspace, sizeof(int32_t), cudaMemcpyDeviceToHost, st))) return R2K_ERR_CUDA;
+  return ok(cudaStreamSynchronize(st)) ? R2K_OK : R2K_ERR_CUDA;
 }
 
 int r2k_merge_states(const float* states, int32_t num_states, int64_t state_stride, int32_t rows, int32_t dtype, void* out,
@@ -724,8 +730,7 @@ int r2k_merge_states(const float* states, int32_t num_states, int64_t state_stri
   if (rc) return rc;
   const cudaError_t err = launch_behind(merge_states_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), reinterpret_cast<cudaStream_t>(stream),
                                         dev->pdl, states, num_states, state_stride, rows, dtype, out, flags);
-  ++g_launches;
-  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(err);
 }
 
 static int check_pack(const void* src, int32_t dtype, int32_t heads, int64_t src_rows, int64_t count, int64_t capacity,
@@ -763,8 +768,7 @@ int r2k_pack_v_int4(const void* src, int32_t dtype, int32_t num_kv_heads, int64_
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (dtype == R2K_DTYPE_BF16) pack_v_int4_kernel<true><<<grid, 128, 0, st>>>(a, packed, scale, 0, 0);
   else pack_v_int4_kernel<false><<<grid, 128, 0, st>>>(a, packed, scale, 0, 0);
-  ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(cudaGetLastError());
 }
 
 int r2k_pack_v_int2(const void* src, int32_t dtype, int32_t num_kv_heads, int64_t src_rows, const int64_t* index, int64_t count,
@@ -790,8 +794,7 @@ int r2k_gather_rows(const void* src, int32_t num_kv_heads, int64_t src_rows, con
   dim3 grid((unsigned)((count + 3) / 4), (unsigned)num_kv_heads, 1);
   gather_rows_kernel<<<grid, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const uint16_t*>(src), src_rows, index, count, reinterpret_cast<uint16_t*>(dst), dst_rows, dst_start);
-  ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(cudaGetLastError());
 }
 
 int r2k_build_cache(const R2KBuild* build, void* stream) {
@@ -851,8 +854,7 @@ int r2k_build_cache(const R2KBuild* build, void* stream) {
   const auto kernel = bf16 ? (other_values ? build_cache_kernel<true, false> : build_cache_kernel<true, true>)
                            : (other_values ? build_cache_kernel<false, true> : build_cache_kernel<false, false>);
   kernel<<<(unsigned)ctas, kBuildThreads, 0, st>>>(a);
-  ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(cudaGetLastError());
 }
 
 int r2k_fwht128(const void* in, void* out, int32_t dtype, int64_t rows, void* stream) {
@@ -868,8 +870,7 @@ int r2k_fwht128(const void* in, void* out, int32_t dtype, int64_t rows, void* st
   if (rc) return rc;
   const cudaError_t err = launch_behind(dtype == R2K_DTYPE_BF16 ? fwht128_kernel<true> : fwht128_kernel<false>, dim3(grid), dim3(128), st, dev->pdl,
                                         reinterpret_cast<const uint16_t*>(in), reinterpret_cast<uint16_t*>(out), rows, wide);
-  ++g_launches;
-  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(err);
 }
 
 int r2k_qk_mrope(const void* q, const void* k, void* q_out, void* k_out, int32_t dtype, int32_t batch, int32_t num_q_heads,
@@ -935,8 +936,7 @@ int r2k_append_recent(const R2KGeom* geom, const R2KCacheView* view, const R2KAp
   append_recent_kernel<<<geom->batch, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       ring_args(geom, view), reinterpret_cast<const uint8_t*>(append->k), reinterpret_cast<const uint8_t*>(append->v),
       append->indices, append->global_index, append->logical_position);
-  ++g_launches;
-  return cudaGetLastError() == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(cudaGetLastError());
 }
 
 int r2k_flush_recent(const R2KGeom* geom, const R2KCacheView* view, int32_t ring_tokens, int32_t flush_tokens, int64_t k_dst,
@@ -985,8 +985,7 @@ int r2k_flush_recent(const R2KGeom* geom, const R2KCacheView* view, int32_t ring
   const cudaError_t err = launch_behind(flush_ring_kernel, dim3((unsigned)geom->batch), dim3(256), st, dev->pdl,
                                         ring_args(geom, view), (int)ring_tokens, (int)flush_tokens, i2_global, i2_logical,
                                         meta_bstride, v_meta_dst);
-  ++g_launches;
-  return err == cudaSuccess ? R2K_OK : R2K_ERR_CUDA;
+  return launched(err);
 }
 
 }  // extern "C"
