@@ -251,3 +251,57 @@ def test_steps_in_a_graph(pages):
         graph.replay()
         for one, other in zip(want, result()):
             assert torch.isfinite(one.float()).all() and torch.equal(other, one)
+
+
+def test_captured_behind_joins_and_copies():
+    """What stands in front of an early launch in a graph: a fill, a copy, two streams that meet, nothing at all."""
+    tokens = 12 * PAGE
+    cache = build_gpu_cache(*random_rows(9, tokens), seeded_classes(12, 9), page_size=PAGE)
+    sharded, rows, side = R.SequenceShardedExecutor(make_executor(cache, HQ)), Rows(31), torch.cuda.Stream()
+    source = [t.clone() for t in rows.rows]
+    turned = torch.zeros(1, HQ, 128, device="cuda", dtype=torch.bfloat16)
+
+    def front(kind):
+        main = torch.cuda.current_stream()
+        if kind == "copy":
+            for t, s in zip(rows.rows, source):
+                t.copy_(s)
+        elif kind == "fill":
+            for t in (*rows.made, sharded.state):
+                t.zero_()
+        elif kind == "join":
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                rows.rows[0].mul_(2)
+            rows.rows[1].mul_(2)
+            main.wait_stream(side)
+
+    def steps():
+        outs = []
+        for kind in ("none", "copy", "join", "fill"):
+            front(kind)
+            q, _, _ = rows.rotate()
+            front(kind)
+            sharded.output = torch.empty(1, HQ, 128, device="cuda", dtype=torch.bfloat16)
+            out = sharded(q)
+            front(kind)
+            outs += [out, R.triton_fwht_128(out, output=turned).clone()]
+        return outs
+
+    def reset():
+        for t, s in zip(rows.rows, source):
+            t.copy_(s)
+        torch.cuda.synchronize()
+
+    reset()
+    want = [t.clone() for t in steps()]
+    reset()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = steps()
+    for _ in range(2):
+        reset()
+        graph.replay()
+        torch.cuda.synchronize()
+        for one, other in zip(want, got):
+            assert torch.isfinite(one.float()).all() and torch.equal(one, other)
