@@ -5,10 +5,10 @@
 // token bookkeeping and set what lies behind the last used row.  Source rows come from the page table (a page's rows are
 // consecutive), so nothing per token is uploaded.
 //
-// Bound by the IEEE divisions (one per key and per quantised value) and the way to them: page search, rows, range, divide.  With
-// 32 rows a warp, keys and values on different warps and one value row at a time, a CTA took 27 us from end to end, and the launch for
-// 32768 tokens x 2 heads 48 us; so 14 and 33.5 us (the rows' bytes alone take 7 us at the copy rate).  With all registers
-// (108 instead of 64, one CTA an SM) 37.5.
+// Bound by the chain through a CTA (page search, rows, range, divide, 14 us from end to end) times its waves: 32768 tokens x 2 heads are
+// 512 CTAs, two on an SM, 1.7 waves, 33.5 us.  The IEEE divisions (one per key and per quantised value) are about 10 us of issue of it,
+// the rows' bytes 7 us at the copy rate.  With 32 rows a warp, keys and values on different warps and one value row at a time, a CTA
+// took 27 us and the launch 48.  64 registers spill 52 to 56 bytes a thread; with all it wants (108, one CTA an SM) the launch takes 37.5.
 #pragma once
 
 #include "pack_kernels.cuh"

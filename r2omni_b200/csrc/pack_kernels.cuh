@@ -382,7 +382,7 @@ __device__ __forceinline__ void split_row(const Row16& r, bool hadamard, float (
 template <bool BF16>
 __global__ void __launch_bounds__(128) fwht128_kernel(const uint16_t* in, uint16_t* out, int64_t rows, bool wide) {
   // launched with programmatic stream serialization: only the way here overlaps the kernel in front (16384 tokens' rotation and values
-  // 47.0 -> 45.2 us)
+  // 45.2 us as an ordinary launch, 44.0 so)
   grid_dependency_wait();
   const int64_t row = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4 + ((threadIdx.x & 31) >> 3);
   const int s = threadIdx.x & 7;
@@ -461,7 +461,8 @@ __global__ void __launch_bounds__(128, 5) mrope_rows_kernel(MropeArgs a) {
   // The decode launch that follows on the stream may start its CTAs and prefetch pool tiles right away (it is
   // launched with programmatic stream serialization); it reads the rows written here only after its own
   // dependency wait, i.e. after this grid has completed.  This kernel itself comes in behind a
-  // projection in the same way (a batch-32 attention block 81.7 -> 78.6 us, the prefill above with its value rows 45.2 -> 43.6).
+  // projection in the same way (a batch-32 attention block 82.5 us as an ordinary launch and 79.8 so, the prefill above with its
+  // value rows 45.6 and 43.7).
   launch_dependents();
   grid_dependency_wait();
   const int s = threadIdx.x & 7;

@@ -170,11 +170,13 @@ int derive(const R2KGeom* g, bool rows, int sms, int clusters, DecodeParams* p) 
   for (int k = 0; k < 4; ++k) head_ns += (double)cnt[k] * ns[k];
   const double per_head = (double)p->grid / p->bh_total;
   // Few heads with few tiles: kCluster CTAs per (request, kv head), one cluster, merge through distributed shared
-  // memory instead of the workspace, which takes 1.3 us off a launch (36 launches of 701 tokens x 2 heads: 300 -> 252 us;
-  // eight of 700 x 8 heads: 74.6 -> 67.5, of 4500 x 8: 97.4 -> 91.8).  Two lines bound it.  Time: fewer CTAs stream longer; eight launches of one
-  // request x 2 heads take 90.2 us without and 76.0 with clusters at 5000 tokens (4.3 us of tile weight more per CTA),
-  // 89.2 and 94.9 at 6500 (6.1 us).  Room: at most two thirds of the clusters that fit, so that some of the next launch's
-  // come in and fetch while this one finishes; 12 heads of 3000 tokens took 88.6 us without and 98.0 with clusters.
+  // memory instead of the workspace, which takes 2.2 us off a launch (36 launches of 701 tokens x 2 heads: 297 -> 220 us;
+  // eight of 700 x 8 heads: 69.1 -> 50.8, of 4500 x 8: 92.0 -> 74.3).  Two lines bound it.  Time: fewer CTAs stream longer; eight launches of one
+  // request x 2 heads take 88.8 us without and 67.6 with clusters at 5000 tokens (4.3 us of tile weight more per CTA),
+  // 90.1 and 75.8 at 6500 (6.1 us), 88.3 and 83.6 at 8000.  Room: at most two thirds of the clusters that fit, so that some of the next
+  // launch's come in and fetch while this one finishes; 12 heads of 3000 tokens take 87.9 us without and 68.1 with clusters.
+  // Both lines were drawn when the merge read its rows out of the other CTAs (94.9 us at 6500 tokens, 98.0 for the 12 heads) and
+  // now lie on the near side of where the two forms meet.
   // The fused exchange merges through the workspace and saves nothing by it, so `rows` has the line of the rule below.
   if (p->grid > p->bh_total && 3 * p->bh_total <= 2 * clusters && kCluster * p->bh_total <= cap && p->c_bh >= (uint32_t)kCluster &&
       head_ns / kCluster - head_ns / per_head < (rows ? 3000.0 : 5000.0)) {
