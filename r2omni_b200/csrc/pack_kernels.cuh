@@ -458,13 +458,14 @@ __device__ __forceinline__ void load_table8(const MropeArgs& a, const void* base
 // heads with the Hadamard in 39 us (151 MB of rows, 3.9 TB/s; 36 us without it), from 139 us with a row per warp.
 template <bool BF16>
 __global__ void __launch_bounds__(128, 5) mrope_rows_kernel(MropeArgs a) {
-  // The decode launch that follows on the stream may start its CTAs and prefetch pool tiles right away (it is
+  // The decode launch that follows on the stream may start its CTAs and prefetch pool tiles early (it is
   // launched with programmatic stream serialization); it reads the rows written here only after its own
-  // dependency wait, i.e. after this grid has completed.  This kernel itself comes in behind a
+  // dependency wait, i.e. after this grid has completed.  It comes in behind this grid's wait: the kernel in front may have written
+  // the pools, and is complete only then.  This kernel itself comes in behind a
   // projection in the same way (a batch-32 attention block 82.5 us as an ordinary launch and 79.8 so, the prefill above with its
   // value rows 45.6 and 43.7).
-  launch_dependents();
   grid_dependency_wait();
+  launch_dependents();
   const int s = threadIdx.x & 7;
   const int64_t n = (int64_t)a.batch * a.tokens;
   const int64_t first = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4;
