@@ -150,6 +150,10 @@ int r2k_decode_plan(const R2KGeom* geom, uint32_t flags, int32_t world, int32_t 
  * to ring row recent_len[b]; recent_len, the two index arrays and the page
  * length are updated on the device.  The ring must have room (host-checked by
  * the caller, as in the reference).
+ * The launch may start when the thread blocks of the kernel in front of it on the stream have exited, and reads
+ * the packed pools before that kernel counts as completed.  This library's writers of the pools provide for it; a
+ * caller's own kernel that writes them, launched directly in front, ends with __threadfence() and does not trigger
+ * programmatic completion before.
  * Replaces SplitKExecutor.__call__ and its three launches
  * (r2omni/sspa/kernels/triton_fourq_splitk.py:1243-1547: _fourq_page_partial_kernel
  * :449-931, _fourq_hierarchical_group_reduce_kernel :1023-1086,

@@ -200,6 +200,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) build_cache_kernel(const __g
     load_rows(b.value, b.rows, head, mine, v);   // on their way beside the keys' arithmetic
     build_keys<BF16>(b, chunk, head, mine, k, range);
     build_values<VALUES_BF16, BF16>(b, chunk, head, mine, v);
+    publish_pools();
     return;
   }
   cta -= a.chunk_ctas;
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) build_cache_kernel(const __g
     for (int i = threadIdx.x; i < words; i += kBuildThreads) reinterpret_cast<uint4*>(p + head_bytes)[i] = make_uint4(v4, v4, v4, v4);
     const int tail = head_bytes + words * 16;
     if (tail + (int)threadIdx.x < bytes) p[tail + threadIdx.x] = (uint8_t)f.value;
+    publish_pools();
     return;
   }
 }

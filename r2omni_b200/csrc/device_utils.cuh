@@ -225,6 +225,10 @@ __device__ __forceinline__ void st_cluster_f4(uint32_t a, float4 v) {
 // (__ldg, const __restrict__) is for memory that nobody writes while the grid runs, and no barrier orders it.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The last thing a thread does that has written the packed pools: a decode launch may come in as soon as this grid's CTAs have left, and
+// reads the pools before its wait for the grid's completion.  Behind the fence they are where it reads them
+// (0.7 of 39 us for a build of 32768 tokens x 2 heads with its page table, queued).
+__device__ __forceinline__ void publish_pools() { __threadfence(); }
 // 16 bytes that are read once; stays behind the wait (both are volatile).
 __device__ __forceinline__ uint4 ld_streamed(const void* p) {
   uint4 v;

@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(64) pack_k_int4_kernel(PackArgs a, uint8_t* pa
   srow[2 * c + 1] = __float2half_rn(st1);
   zrow[2 * c] = (uint8_t)zp0;
   zrow[2 * c + 1] = (uint8_t)zp1;
+  if (!a.in_flush) publish_pools();   // a flush's last launch waits for this grid
 }
 
 // ---- values: one warp per (token, head, request), lane owns dims 4l..4l+3 ---
@@ -174,6 +175,7 @@ __global__ void __launch_bounds__(128) pack_v_int4_kernel(PackArgs a, uint8_t* p
   const int64_t row = (int64_t)head * a.capacity + a.dst_start + i;
   *reinterpret_cast<uint16_t*>(packed + req * packed_bstride + row * 64 + 2 * lane) = out;
   if (lane == 0) *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(scale) + req * scale_bstride + row * 4) = sc;
+  publish_pools();
 }
 
 template <bool BF16>
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(128) pack_v_int2_kernel(PackArgs a, uint8_t* p
       reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(scale) + req * scale_bstride)[m] = __float2half_rn(sc);
       zero[req * zero_bstride + m] = (uint8_t)zp;
     }
+    if (!a.in_flush) publish_pools();   // a flush's last launch waits for this grid
   }
   // In a flush this grid runs beside the key pack in front of it.  The ring kernel behind it waits for this
   // grid only, so this grid must not complete before the key pack has: every thread passes here on its way out.
@@ -212,6 +215,7 @@ __global__ void __launch_bounds__(128) gather_rows_kernel(const uint16_t* src, i
   const int64_t s = index ? index[i] : i;
   const uint2 w = *reinterpret_cast<const uint2*>(src + ((int64_t)head * src_rows + s) * 128 + 4 * lane);
   *reinterpret_cast<uint2*>(dst + ((int64_t)head * dst_rows + dst_start + i) * 128 + 4 * lane) = w;
+  publish_pools();
 }
 
 // ---- host block copy ---------------------------------------------------------

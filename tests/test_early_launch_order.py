@@ -25,3 +25,12 @@ def test_who_lets_the_next_launch_in():
         assert "launch_dependents" not in bodies[name]
     for name in ("pack_k_int4_kernel", "pack_v_int2_kernel"):   # in a flush alone: its last launch waits for both
         assert re.findall(r"[^;{}]*launch_dependents\(\)", bodies[name])[0].strip() == "if (a.in_flush) launch_dependents()"
+
+
+def test_pool_writers_publish_what_they_wrote():
+    """A decode launch behind one of them may come in when its CTAs have left, before the grid counts as completed."""
+    bodies = dict(kernels())
+    for name in ("pack_k_int4_kernel", "pack_v_int4_kernel", "pack_v_int2_kernel", "gather_rows_kernel"):
+        assert bodies[name].count("publish_pools()") == 1, name
+    build = bodies["build_cache_kernel"]   # its rows and its fills; the token bookkeeping is not read by a decode launch
+    assert re.search(r"build_values<[^;]*;\s*publish_pools\(\);\s*return;", build) and build.rstrip().endswith("publish_pools();\n    return;\n  }")

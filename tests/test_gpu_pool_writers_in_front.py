@@ -305,3 +305,29 @@ def test_captured_behind_joins_and_copies():
         torch.cuda.synchronize()
         for one, other in zip(want, got):
             assert torch.isfinite(one.float()).all() and torch.equal(one, other)
+
+
+@pytest.mark.parametrize("pages", [12, 700])
+def test_decode_directly_behind_a_build(pages):
+    """No launch in between: each cache takes the memory of the one before it."""
+    tokens, steps = pages * PAGE, 6
+    plan = _plan(seeded_classes(pages, 3), [PAGE] * pages)
+    sources, q = [random_rows(s, tokens) for s in (1, 2)], Rows(3).rows[0]
+    ws = R.allocate_splitk_workspace(R.build_three_precision_cache(*sources[1], plan, page_size=PAGE), num_query_heads=HQ)
+
+    def run(wait):
+        outs = torch.zeros(steps, 1, HQ, 130, device="cuda")
+        queue(wait)
+        for i in range(steps):
+            ex = cache = None
+            cache = R.build_three_precision_cache(*sources[i % 2], plan, page_size=PAGE)
+            settle(wait)
+            ex = R.prepare_splitk_executor(cache, ws)
+            ex.decode_state(q, out=outs[i])
+            settle(wait)
+        torch.cuda.synchronize()
+        return outs
+
+    want = run(True)
+    assert torch.isfinite(want).all() and not torch.equal(want[0], want[1])
+    assert torch.equal(run(False), want)
